@@ -248,3 +248,48 @@ def tolerance(case):
     if kind == "linear":
         return {"rel": 7e-3}
     return "exact"
+
+
+def _e4m3_groups(x):
+    """x [rows, cols] bf16 in the wire format, e4m3 with one fp32 scale per 128 elements, as the fp64 values it stands for.
+    The format is part of the path's definition, so the 64-bit results start from its values."""
+    g = x.float().reshape(x.shape[0], -1, 128)
+    amax = g.abs().amax(dim=-1, keepdim=True).clamp_min(1e-4)
+    top = torch.full_like(amax, 448.0)
+    q = (g * (top / amax)).clamp(-448.0, 448.0).to(torch.float8_e4m3fn)
+    return (q.double() * (amax / top).double()).reshape(x.shape)
+
+
+def exact(case, seed):
+    """What ``run`` returns for these inputs in 64-bit arithmetic, without the bf16 roundings on the way; ``None`` for
+    what is only moved."""
+    kind = case["kind"]
+    if kind not in ("moe", "linear", "prefill"):
+        return None
+    st = prepare(case, seed)
+    if kind == "linear":
+        if case["dtype"] == "bf16":
+            return st["x"].double() @ st["w"].double().t()
+        q, s = st["w"]
+        blocks = s.double().repeat_interleave(128, 0)[: case["n"]].repeat_interleave(128, 1)[:, : case["k"]]
+        return _e4m3_groups(st["x"]) @ (q.double() * blocks).t()
+    if kind == "prefill":
+        a = st["hidden"].double()
+        weights = [w.double() for w in st["weights"]]
+        for layer in range(case["layers"]):
+            a = a @ weights[layer % len(weights)].t()
+        return a, None, None
+    layer, inter = st["layer"], case["inter"]
+    gates, picked = torch.topk(torch.softmax(st["logits"].double(), dim=-1), case["topk"], dim=-1)
+    if case["renormalize"]:
+        gates = gates / gates.sum(-1, keepdim=True)
+    x = _e4m3_groups(st["x"])
+    out = torch.zeros_like(x)
+    for e in range(case["experts"]):
+        tok, k = (picked == e).nonzero(as_tuple=True)
+        if tok.numel() == 0:
+            continue
+        gate_up = x[tok] @ layer.w_gate_up[e].double().t()
+        h = torch.nn.functional.silu(gate_up[:, :inter]) * gate_up[:, inter:]
+        out.index_add_(0, tok, gates[tok, k].unsqueeze(1) * (h @ layer.w_down[e].double().t()))
+    return out
