@@ -10,11 +10,17 @@
 // source (pack, or prefill -> decode transfer when the paged side is a peer's cache);
 // otherwise the paged side is the source (unpack).
 //
-// One launch moves K and V of one layer for the whole batch: CTAs walk (task, plane)
-// units and copy with 16-byte vectors, eight in flight per thread. The last CTA to finish
-// publishes `done_value` at `done_flag` (release, system scope), typically a per-layer
+// One launch moves K and V of one layer for the whole batch: warps walk 4 KB slices of the (task, plane) pages.
+// The last CTA to finish publishes `done_value` at `done_flag` (release, system scope), typically a per-layer
 // word in the decode rank's memory, so the consumer can start attention on layer l while
 // layer l+1 is still in flight.
+//
+// A transfer that runs beside the prefill GEMMs gets few CTAs (32 by default) without shared memory, so its rate is
+// the bytes that those CTAs keep in flight over the memory latency. Every warp has a slice being stored, the next one on
+// its way and the page header of the one after that, whatever the page size. (With one page per CTA at a time, its
+// header fetched when the CTA came to it, nothing was in flight between two pages: 30 MB per layer, 32 CTAs, 64-token pages of 512-byte
+// rows took 55 us a layer where this takes 42 us, and 4 KB pages left most of a CTA idle. With 148 CTAs it is 20 us,
+// 2.9 TB/s read and written.)
 #include "common/host_utils.h"
 #include "common/ptx.cuh"
 #include "slime_cuda.h"
@@ -41,38 +47,90 @@ struct KvArgs {
     KernelStatus*       status;
 };
 
+constexpr int kSliceVecs = 8;                      // 16-byte vectors per lane and slice
+constexpr int kSliceSpan = 32 * kSliceVecs;        // vectors of a slice: 4 KB
+
+// One slice of one page: where it lies and how many of this lane's vectors exist.
+struct KvSlice {
+    const uint4* src;
+    uint4*       dst;
+    int          left;  // vectors from this lane's first one to the end of the page; lane's j-th exists if 32 * j < left
+};
+
+struct KvHeader {
+    int toff, blk, n;
+};
+
+__device__ __forceinline__ KvHeader kv_header(const KvArgs& a, int p)
+{
+    return {a.tok_off[p], a.blk[p], a.ntok ? a.ntok[p] : a.page_tokens};
+}
+
+// Resolves item -> slice. An item of a short page that lies past the page's end, or whose task is out of range (reported
+// once), moves nothing.
+__device__ __forceinline__ KvSlice kv_slice(const KvArgs& a, KvHeader h, long long item, int slices, int lane)
+{
+    const long long u     = item / slices;
+    const int       slice = static_cast<int>(item - u * slices);
+    const int       p     = static_cast<int>(u >> 1);
+    const int       plane = static_cast<int>(u & 1);
+    KvSlice         s{nullptr, nullptr, 0};
+    if (h.n > a.page_tokens) h.n = a.page_tokens;
+    if (h.n <= 0) return s;
+    if (h.toff < 0 || static_cast<unsigned long long>(h.toff) + h.n > a.tok_rows || h.blk < 0
+        || static_cast<unsigned long long>(h.blk) >= a.page_blocks) {
+        if (lane == 0 && slice == 0) report_status(a.status, K_BAD_INDEX, 80, p, a.page_blocks, static_cast<unsigned long long>(h.blk));
+        return s;
+    }
+    const unsigned long long tok_addr  = (plane ? a.tok_v : a.tok_k) + static_cast<unsigned long long>(h.toff) * a.row_bytes;
+    const unsigned long long page_addr = (plane ? a.page_v : a.page_k) + static_cast<unsigned long long>(h.blk) * a.page_tokens * a.row_bytes;
+    const long long          first     = static_cast<long long>(slice) * kSliceSpan + lane;
+    const long long          left      = static_cast<long long>(static_cast<unsigned long long>(h.n) * a.row_bytes / 16) - first;
+    s.src  = reinterpret_cast<const uint4*>(a.to_paged ? tok_addr : page_addr) + first;
+    s.dst  = reinterpret_cast<uint4*>(a.to_paged ? page_addr : tok_addr) + first;
+    s.left = left <= 0 ? 0 : left > kSliceSpan ? kSliceSpan : static_cast<int>(left);
+    return s;
+}
+
+__device__ __forceinline__ void kv_load(const KvSlice& s, uint4 (&v)[kSliceVecs])
+{
+#pragma unroll
+    for (int j = 0; j < kSliceVecs; ++j)
+        if (32 * j < s.left) v[j] = s.src[32 * j];
+}
+
+__device__ __forceinline__ void kv_store(const KvSlice& s, const uint4 (&v)[kSliceVecs])
+{
+#pragma unroll
+    for (int j = 0; j < kSliceVecs; ++j)
+        if (32 * j < s.left) s.dst[32 * j] = v[j];
+}
+
 __global__ void __launch_bounds__(256) kv_transfer_kernel(KvArgs a)
 {
-    const long long units = 2ll * a.n_tasks;
-    for (long long u = blockIdx.x; u < units; u += gridDim.x) {
-        const int p     = static_cast<int>(u >> 1);
-        const int plane = static_cast<int>(u & 1);
-        const int toff  = a.tok_off[p];
-        const int b     = a.blk[p];
-        int       n     = a.ntok ? a.ntok[p] : a.page_tokens;
-        if (n > a.page_tokens) n = a.page_tokens;
-        if (n <= 0) continue;
-        if (toff < 0 || static_cast<unsigned long long>(toff) + n > a.tok_rows || b < 0
-            || static_cast<unsigned long long>(b) >= a.page_blocks) {
-            if (threadIdx.x == 0) report_status(a.status, K_BAD_INDEX, 80, p, a.page_blocks, static_cast<unsigned long long>(b));
-            continue;
-        }
-        const unsigned long long tok_addr  = (plane ? a.tok_v : a.tok_k) + static_cast<unsigned long long>(toff) * a.row_bytes;
-        const unsigned long long page_addr = (plane ? a.page_v : a.page_k)
-                                             + static_cast<unsigned long long>(b) * a.page_tokens * a.row_bytes;
-        const uint4* src = reinterpret_cast<const uint4*>(a.to_paged ? tok_addr : page_addr);
-        uint4*       dst = reinterpret_cast<uint4*>(a.to_paged ? page_addr : tok_addr);
-        const unsigned long long nv = static_cast<unsigned long long>(n) * a.row_bytes / 16;
-        const unsigned long long nt = blockDim.x;
-        unsigned long long       i  = threadIdx.x;
-        for (; i + 7ull * nt < nv; i += 8ull * nt) {
-            uint4 v[8];
-#pragma unroll
-            for (int j = 0; j < 8; ++j) v[j] = src[i + j * nt];
-#pragma unroll
-            for (int j = 0; j < 8; ++j) dst[i + j * nt] = v[j];
-        }
-        for (; i < nv; i += nt) dst[i] = src[i];
+    const int       lane   = threadIdx.x & 31;
+    const int       warps  = blockDim.x >> 5;
+    const int       slices = static_cast<int>((a.page_tokens * a.row_bytes / 16 + kSliceSpan - 1) / kSliceSpan);
+    const long long items  = 2ll * a.n_tasks * slices;
+    const long long step   = static_cast<long long>(gridDim.x) * warps;
+    long long       item   = static_cast<long long>(blockIdx.x) * warps + (threadIdx.x >> 5);
+    // Two slices per warp are in flight at any time, and the page header of the one after them.
+    auto header = [&](long long i) { return i < items ? kv_header(a, static_cast<int>(i / slices >> 1)) : KvHeader{0, 0, 0}; };
+    auto resolve = [&](const KvHeader& h, long long i) { return i < items ? kv_slice(a, h, i, slices, lane) : KvSlice{nullptr, nullptr, 0}; };
+    uint4    v0[kSliceVecs], v1[kSliceVecs];
+    KvHeader h0 = header(item), h1 = header(item + step);
+    KvSlice  s0 = resolve(h0, item), s1;
+    kv_load(s0, v0);
+    while (item < items) {
+        h0 = header(item + 2 * step);
+        s1 = resolve(h1, item + step);
+        kv_load(s1, v1);
+        kv_store(s0, v0);
+        h1 = header(item + 3 * step);
+        s0 = resolve(h0, item + 2 * step);
+        kv_load(s0, v0);
+        kv_store(s1, v1);
+        item += 2 * step;
     }
     if (a.done_flag != nullptr) {
         __shared__ bool is_last;
@@ -124,7 +182,10 @@ int slime_kv_transfer(unsigned long long tok_k, unsigned long long tok_v, unsign
     a.done_value    = done_value;
     a.block_counter = block_counter;
     a.status        = static_cast<KernelStatus*>(status);
-    long long grid = 2ll * n_tasks;
+    const unsigned long long slices = (static_cast<unsigned long long>(page_tokens) * row_bytes / 16 + kSliceSpan - 1) / kSliceSpan;
+    if (slices > 0x7fffffffull) return fail("kv transfer: a page of %d rows of %llu bytes is too large", page_tokens, row_bytes);
+    const long long warps = g_kv_threads / 32;
+    long long       grid  = (2ll * n_tasks * static_cast<long long>(slices) + warps - 1) / warps;
     const long long cap = max_blocks > 0 ? max_blocks : sm_count() * 4;
     if (grid > cap) grid = cap;
     if (grid < 1) grid = 1;

@@ -81,3 +81,34 @@ def test_prefill_sender_pushes_every_layer_with_flags():
     got = cache.tensor()
     for t, b, n in zip(tok_off.tolist(), blk.tolist(), ntok.tolist()):
         assert torch.equal(got[:, :, b, :n], sender.kv_stage[:, :, t:t + n])
+
+
+@pytest.mark.parametrize("page,row,lens,threads", [(1, 8, [5, 1], 256), (7, 2056, [7, 20, 1], 256), (16, 128, [1000, 16, 3], 32), (64, 512, [63, 65, 640], 96)])
+def test_page_sizes_that_are_no_multiple_of_a_slice(page, row, lens, threads):
+    """Pages below, above and beside the 4 KB slices that a warp moves, from a page of 16 bytes on; short last pages, CTAs of
+    one, three and eight warps, fewer CTAs than slices; nothing outside the pages' rows is written."""
+    from dlslime_b200.ops import kv
+    from dlslime_b200.ops._common import default_status
+
+    (tok_off, blk, ntok), _, blocks = _setup(lens, page, row)
+    total, rb = sum(lens), row * 2
+    src = torch.randn(2, total, row, device="cuda").to(torch.bfloat16)
+    paged = torch.full((2, blocks, page, row), 3.0, device="cuda", dtype=torch.bfloat16)
+    expect = paged.clone()
+    for t, b, n in zip(tok_off.tolist(), blk.tolist(), ntok.tolist()):
+        expect[:, b, :n] = src[:, t:t + n]
+    back = torch.full_like(src, 4.0)
+    kv.tune(threads)
+    try:
+        for max_blocks in (0, 3):
+            kv.kv_move(src[0].data_ptr(), src[1].data_ptr(), paged[0].data_ptr(), paged[1].data_ptr(), tok_off, blk, ntok,
+                       page_tokens=page, row_bytes=rb, tok_rows=total, page_blocks=blocks, to_paged=True, max_blocks=max_blocks)
+            kv.kv_move(back[0].data_ptr(), back[1].data_ptr(), paged[0].data_ptr(), paged[1].data_ptr(), tok_off, blk, ntok,
+                       page_tokens=page, row_bytes=rb, tok_rows=total, page_blocks=blocks, to_paged=False, max_blocks=max_blocks)
+            torch.cuda.synchronize()
+            default_status().check()
+            assert torch.equal(paged, expect) and torch.equal(back, src)
+            paged.fill_(3.0)
+            back.fill_(4.0)
+    finally:
+        kv.tune(256)
