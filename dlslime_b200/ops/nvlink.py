@@ -25,7 +25,7 @@ from typing import Sequence
 import numpy as np
 import torch
 
-from .. import _lib
+from .. import _lib, _slime_c
 from ._common import stream_ptr
 
 _v, _i, _ull, _cp = ctypes.c_void_p, ctypes.c_int, ctypes.c_ulonglong, ctypes.c_char_p
@@ -107,8 +107,6 @@ class NVLinkEndpoint:
         # Accounting (DLSLIME_OBS=1): this endpoint is one link of kind "nvlink" in the process's counters, with the same
         # submit / complete semantics per user operation as the RDMA links. Off: one `is None` test per transfer.
         self._obs_link = None
-        from .. import _slime_c
-
         if _slime_c.obs_enabled():
             self._obs = _slime_c
             self._obs_link = _slime_c.obs_register_link(f"nvlink:gpu{torch.cuda.current_device()}", "nvlink")
@@ -186,6 +184,10 @@ class NVLinkEndpoint:
                     raise KeyError(f"memory region not found: local={ln!r} remote={rn!r}")
                 rows.append((lh, rh, roff, loff, length))
             assign = rows
+        arr = np.empty((len(assign), 5), dtype=np.uint64)
+        bad = _slime_c._pack_assignment_rows(assign, arr.ctypes.data)
+        if bad == -1:
+            return arr
         for row in assign:
             if min(int(v) for v in row) < 0:
                 raise ValueError(f"negative handle, offset or length in assignment {tuple(row)!r}")

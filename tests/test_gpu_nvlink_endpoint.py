@@ -158,3 +158,37 @@ def test_transfers_are_accounted_as_an_nvlink_link():
     finally:
         _slime_c.obs_reset_for_test()
         _slime_c.obs_set_enabled_for_test(False)
+
+
+@pytest.mark.parametrize("count", [8, 9, 100, 101, 400])
+def test_pieces_at_every_misalignment(pair, count):
+    """Pieces whose source and destination sit at every offset inside 16 bytes, of every short length and of some long ones,
+    in batches around the sizes at which they travel as kernel arguments or as a table; bytes between the pieces stay."""
+    ep, mine, theirs = pair
+    lh, rh = ep.get_mr_handle("buf"), ep.get_remote_mr_handle("buf")
+    segs, at = [], 0
+    for i in range(count):
+        j = i * 37  # walks through all 256 pairs of offsets
+        n = (j % 50) if i % 4 else 1000 + 977 * (i % 70)
+        segs.append((at + 64 + j % 16, at + 64 + (j // 16) % 16, n))
+        at += 128 + n
+    expect = mine.clone()
+    _apply(expect, theirs, segs, False)
+    assert ep.read([(lh, rh, roff, loff, n) for roff, loff, n in segs]).wait(10.0) == 0
+    assert torch.equal(mine, expect)
+
+
+def test_assignments_that_are_not_plain_integers(pair):
+    """Rows as lists, numpy integers and mixed with tuples take the general path to the same result."""
+    import numpy as np
+
+    ep, mine, theirs = pair
+    lh, rh = ep.get_mr_handle("buf"), ep.get_remote_mr_handle("buf")
+    rows = [(lh, rh, 1000 * i, 500 * i, 300) for i in range(12)]
+    expect = mine.clone()
+    _apply(expect, theirs, [r[2:] for r in rows], False)
+    for batch in ([list(r) for r in rows], [tuple(np.int64(v) for v in r) for r in rows], tuple(rows), np.asarray(rows, dtype=np.uint64)):
+        mine.copy_(expect)
+        mine[:6000] = 0
+        assert ep.read(batch).wait(10.0) == 0
+        assert torch.equal(mine[:300], expect[:300]) and torch.equal(mine[5500:5800], expect[5500:5800])
