@@ -140,6 +140,9 @@ int slime_ep_route(const void* cfg_bytes, const float* logits, int T, int* topk_
 int slime_ep_dispatch(const void* cfg_bytes, const void* x, long long ldx, int T, const int* topk_idx, const int* slot,
                       int* group_offsets, unsigned int* block_counter, unsigned long long epoch, int max_blocks,
                       void* status, void* stream);
+int slime_ep_dispatch_expand(const void* cfg_bytes, const void* x, long long ldx, int T, const int* topk_idx, const int* slot,
+                             int* group_offsets, unsigned int* block_counter, void* y, long long ldy, unsigned long long epoch,
+                             int max_blocks, void* status, void* stream);
 // Streamed form (rows pushed expert by expert, one arrival word per source rank and local expert, so that the
 // receive side and the grouped GEMM start while later experts are still in flight):
 //   route_ordered    route + push_off [num_experts + 1]: start of each expert's rows in this rank's push order

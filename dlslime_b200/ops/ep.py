@@ -237,6 +237,16 @@ class EpBuffer:
                   ptr(self.group_offsets), self._bc1, e, max_blocks,
                   self.status.dev_ptr, stream_ptr())
 
+    def dispatch_expand(self, x: torch.Tensor, out: torch.Tensor, epoch: int | None = None, max_blocks: int = 0) -> None:
+        """:meth:`dispatch` and :meth:`recv_dequant` in one pass, for a buffer of one rank: the bf16 rows that the receive
+        would make of the quantised ones go straight to ``out`` [recv_cap, hidden]; ``recv_x`` / ``recv_scale`` are not written."""
+        T = x.shape[0]
+        assert x.dtype == torch.bfloat16 and x.stride(1) == 1 and x.shape[1] == self.hidden
+        assert out.dtype == torch.bfloat16 and out.stride(1) == 1 and out.shape == (self.recv_cap, self.hidden)
+        cfg, e = self._mode(epoch)
+        _lib.call("slime_ep_dispatch_expand", cfg, ptr(x), x.stride(0), T, ptr(self.topk_idx), ptr(self.slot),
+                  ptr(self.group_offsets), self._bc1, ptr(out), out.stride(0), e, max_blocks, self.status.dev_ptr, stream_ptr())
+
     # -- streamed form ------------------------------------------------------------------
     def route_ordered(self, logits: torch.Tensor | None, T: int, epoch: int | None = None, renormalize: bool = False) -> None:
         """``route`` that also lays out this rank's push order (expert by expert) for ``dispatch_ordered``."""
@@ -331,6 +341,7 @@ import ctypes as _ct  # noqa: E402
 _v, _i, _ll, _ull = _ct.c_void_p, _ct.c_int, _ct.c_longlong, _ct.c_ulonglong
 _lib.declare("slime_ep_route", [_ct.c_char_p, _v, _i, _v, _v, _v, _v, _v, _ull, _i, _v])
 _lib.declare("slime_ep_dispatch", [_ct.c_char_p, _v, _ll, _i, _v, _v, _v, _v, _ull, _i, _v, _v])
+_lib.declare("slime_ep_dispatch_expand", [_ct.c_char_p, _v, _ll, _i, _v, _v, _v, _v, _v, _ll, _ull, _i, _v, _v])
 _lib.declare("slime_ep_route_ordered", [_ct.c_char_p, _v, _i, _v, _v, _v, _v, _v, _ull, _i, _v, _v])
 _lib.declare("slime_ep_layout", [_ct.c_char_p, _v, _ull, _v, _v])
 _lib.declare("slime_ep_dispatch_ordered", [_ct.c_char_p, _v, _v, _i, _v, _v, _v, _v, _v, _ull, _i, _v, _v])

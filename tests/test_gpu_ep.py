@@ -243,3 +243,39 @@ def test_device_trace_counts_rows_and_waits():
     bufs[0].enable_device_trace(False)
     with pytest.raises(RuntimeError):
         bufs[0].device_trace()
+
+
+@pytest.mark.parametrize("tokens,hidden,ldx", [(1, 512, 512), (37, 1536, 1544), (300, 7168, 7168)])
+def test_dispatch_expand_writes_what_dispatch_and_receive_do(tokens, hidden, ldx):
+    """One rank: the pass that writes the expanded rows at once against dispatch followed by the receive, bit for bit, with
+    rows of zeros, tokens that skip some of their experts and a pitch wider than the row."""
+    from dlslime_b200.ops._common import default_status
+    from dlslime_b200.ops.ep import EpBuffer
+
+    experts, topk = 16, 4
+    buf = EpBuffer(experts, topk, hidden, tokens)
+    gen = torch.Generator(device="cuda").manual_seed(tokens)
+    x = torch.zeros((tokens, ldx), device="cuda", dtype=torch.bfloat16)[:, :hidden]
+    x.copy_(torch.randn((tokens, hidden), generator=gen, device="cuda") * 3)
+    x[tokens // 2] = 0
+    idx = torch.rand((tokens, experts), generator=gen, device="cuda").topk(topk).indices.to(torch.int32)
+    idx[:, 1] = torch.where(torch.arange(tokens, device="cuda") % 3 == 0, -1, idx[:, 1])
+    got = {}
+    for form in ("two passes", "one pass"):
+        buf.topk_idx.copy_(idx)
+        y = torch.full((buf.recv_cap, hidden), 5.0, device="cuda", dtype=torch.bfloat16)
+        buf.route(None, tokens, None)
+        if form == "one pass":
+            buf.dispatch_expand(x, y, None)
+        else:
+            buf.dispatch(x, None)
+            buf.recv_dequant(y, None, tokens * topk)
+        torch.cuda.synchronize()
+        default_status().check()
+        rows = int(buf.group_offsets[-1])
+        assert rows == int((idx >= 0).sum()) and (y[rows:] == 5.0).all()
+        # rows of one expert come in the order of the slot counters, which differs from run to run
+        order = torch.argsort(buf.recv_info[:rows])
+        got[form] = (buf.group_offsets.clone(), buf.recv_info[:rows][order].clone(), y[:rows][order].clone())
+    for a, b in zip(*got.values()):
+        assert torch.equal(a, b)
