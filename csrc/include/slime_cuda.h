@@ -96,6 +96,12 @@ int slime_grouped_gemm_bf16_tile(const void* A, const void* B, void* C, const in
                                  const void* row_info, const unsigned long long* scatter_bases8,
                                  unsigned long long scatter_row_bytes, unsigned long long scatter_slots,
                                  const float* row_scale, int tile_n, int w_prefetch, int tile_m, void* status, void* stream);
+// Weights on the M side, at most tile_tokens (64 / 128 / 192) rows of a group per tile: for launches that stream weights.
+int slime_grouped_gemm_bf16_wt(const void* A, const void* B, void* C, const int* group_offsets, int num_groups,
+                               int M_cap, int N, int K, long long lda, long long ldb, long long ldc, int epilogue,
+                               const void* row_info, const unsigned long long* scatter_bases8,
+                               unsigned long long scatter_row_bytes, unsigned long long scatter_slots,
+                               const float* row_scale, int tile_tokens, int chained, void* status, void* stream);
 // The same on CTA pairs (clusters of two CTAs, 256-row tiles): faster where groups hold several hundred rows or more.
 int slime_grouped_gemm_bf16_pair(const void* A, const void* B, void* C, const int* group_offsets, int num_groups,
                                  int M_cap, int N, int K, long long lda, long long ldb, long long ldc, int epilogue,

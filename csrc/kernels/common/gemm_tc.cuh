@@ -83,6 +83,9 @@ struct Args {
     // rows: 5.52 against 5.02 and less): 148 CTAs with four 48 KB stages already keep HBM busy, and the extra requests
     // only disturb the order in which it is read. Off everywhere; kept as an option of the launcher.
     int                       w_prefetch;
+    // programmatic launch behind the kernel in front of it in the stream (gemm_wt.cuh): 1 = everything waits for that kernel's
+    // completion after the set-up, 2 = the group offsets and B are older than that kernel
+    int                       chained;
     // A operand as e4m3 with 1x128 scales (kernels instantiated with A8): the tile is expanded to bf16 in shared memory
     const float*              a_scale;         // [M_total, K / 128]
     KernelStatus*             status;

@@ -4,6 +4,7 @@
 // weighted rows to arbitrary (possibly peer) addresses.
 #include "common/gemm_tc2s.cuh"
 #include "common/gemm_tc2w.cuh"
+#include "common/gemm_wt.cuh"
 #include "common/host_utils.h"
 #include "slime_cuda.h"
 
@@ -256,6 +257,41 @@ int launch_pair_wide(const void* A, const void* B, const Args& args, long long l
     return 0;
 }
 
+// Weights on the M side, the tokens of a group on the N side (gemm_wt.cuh).
+template<int PTOK, int EPI>
+int launch_wt(const void* A, const void* B, const Args& args, long long lda, long long ldb, cudaStream_t stream)
+{
+    using S = SmemWt<PTOK>;
+    CUtensorMap tmW, tmX32, tmX16;
+    const unsigned long long rowsB_total = static_cast<unsigned long long>(args.rowsB) * args.num_groups;
+    if (make_tmap_2d(&tmW, B, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, rowsB_total, args.K, ldb, 128, kBK)) return -1;
+    if (make_tmap_2d(&tmX32, A, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, args.M_total, args.K, lda, 32, kBK)) return -1;
+    if (make_tmap_2d(&tmX16, A, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, args.M_total, args.K, lda, 16, kBK)) return -1;
+    auto kern = gemm_bf16_wt_kernel<PTOK, EPI>;
+    static bool configured = false;
+    if (!configured) {
+        SLIME_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, S::kTotal));
+        configured = true;
+    }
+    if (args.chained) {
+        SLIME_CUDA_OK(launch_programmatic(kern, dim3(sm_count()), dim3(kWtThreads), S::kTotal, stream, tmW, tmX32, tmX16, args));
+        return 0;
+    }
+    kern<<<sm_count(), kWtThreads, S::kTotal, stream>>>(tmW, tmX32, tmX16, args);
+    SLIME_CUDA_OK(cudaGetLastError());
+    return 0;
+}
+
+template<int EPI>
+int launch_wt(int max_tokens, const void* A, const void* B, const Args& args, long long lda, long long ldb, cudaStream_t stream)
+{
+    switch (max_tokens) {
+        case 64: return launch_wt<64, EPI>(A, B, args, lda, ldb, stream);
+        case 128: return launch_wt<128, EPI>(A, B, args, lda, ldb, stream);
+        default: return launch_wt<192, EPI>(A, B, args, lda, ldb, stream);
+    }
+}
+
 int check_common(int M, int N, int K, long long lda, long long ldb)
 {
     if (M <= 0 || N <= 0 || K <= 0) return fail("gemm: M, N, K must be positive (got %d, %d, %d)", M, N, K);
@@ -406,6 +442,8 @@ static int grouped_gemm_impl(const void* A, const void* B, void* C, const int* g
                             void* status, void* stream);
 static thread_local unsigned long long* g_group_trace  = nullptr;  // set around one traced launch
 static thread_local unsigned int*       g_tile_counter = nullptr;
+static thread_local int                 g_wt_tokens    = 0;  // set around one launch with the weights on the M side: tokens per tile
+static thread_local int                 g_chained      = 0;  // and whether it is chained to the kernel in front of it (Args::chained)
 static thread_local int                 g_on_pairs     = 0;  // set around one launch on CTA pairs: 1 = 256 x 256 tiles, 2 = 256 x 512
 int slime_grouped_gemm_bf16_gated_traced(const void* A, const void* B, void* C, const int* group_offsets, int num_groups,
                                          int M_cap, int N, int K, long long lda, long long ldb, long long ldc, int epilogue,
@@ -445,6 +483,30 @@ int slime_grouped_gemm_bf16_tile(const void* A, const void* B, void* C, const in
     g_tile_n     = 0;
     g_w_prefetch = 0;
     g_tile_m     = 0;
+    return rc;
+}
+
+// The same for launches that stream weights (up to a few hundred rows per group): weights on the M side, tiles of 256
+// weight rows by at most `tile_tokens` (64, 128 or 192) rows of a group; larger groups are cut into equal parts. chained:
+// 0, or the launch is scheduled while the kernel in front of it in the stream drains: 1 = it touches nothing before that
+// kernel has completed, 2 = the group offsets and B were written before that kernel began, and the first weights are
+// fetched at once.
+int slime_grouped_gemm_bf16_wt(const void* A, const void* B, void* C, const int* group_offsets, int num_groups,
+                               int M_cap, int N, int K, long long lda, long long ldb, long long ldc, int epilogue,
+                               const void* row_info, const unsigned long long* scatter_bases8,
+                               unsigned long long scatter_row_bytes, unsigned long long scatter_slots,
+                               const float* row_scale, int tile_tokens, int chained, void* status, void* stream)
+{
+    if (tile_tokens != 64 && tile_tokens != 128 && tile_tokens != 192) return fail("grouped gemm: tiles of %d tokens are not offered", tile_tokens);
+    if (chained < 0 || chained > 2) return fail("grouped gemm: chained = %d not in [0, 2]", chained);
+    if (epilogue != kEpiScatterRows && (ldc % 8 != 0 || (reinterpret_cast<unsigned long long>(C) & 15) != 0))
+        return fail("grouped gemm: rows of the output must be 16-byte aligned");
+    g_wt_tokens  = tile_tokens;
+    g_chained    = chained;
+    const int rc = grouped_gemm_impl(A, B, C, group_offsets, num_groups, M_cap, N, K, lda, ldb, ldc, epilogue, row_info, scatter_bases8,
+                                     scatter_row_bytes, scatter_slots, row_scale, nullptr, 0, nullptr, status, stream);
+    g_wt_tokens  = 0;
+    g_chained    = 0;
     return rc;
 }
 
@@ -545,6 +607,7 @@ static int grouped_gemm_impl(const void* A, const void* B, void* C, const int* g
     a.group_trace        = g_group_trace;
     a.tile_counter       = g_tile_counter;
     a.w_prefetch         = g_w_prefetch;
+    a.chained            = g_chained;
     a.M_total       = M_cap;
     a.N             = N;
     a.K             = K;
@@ -557,12 +620,14 @@ static int grouped_gemm_impl(const void* A, const void* B, void* C, const int* g
     switch (epilogue) {
         case kEpiStore:
             a.rowsB = N;
+            if (g_wt_tokens) return launch_wt<kEpiStore>(g_wt_tokens, A, B, a, lda, ldb, s);
             return g_on_pairs == 3 ? launch_pair_swapped<kEpiStore>(A, B, a, lda, ldb, s)
                    : g_on_pairs == 2 ? launch_pair_wide<kEpiStore>(A, B, a, lda, ldb, s)
                    : g_on_pairs ? launch_pair_grouped<kEpiStore>(A, B, a, lda, ldb, s) : launch<kEpiStore>(A, B, a, lda, ldb, s);
         case kEpiSwiGLU:
             if (N % 32 != 0) return fail("grouped gemm: SwiGLU needs N to be a multiple of 32");
             a.rowsB = 2 * N;
+            if (g_wt_tokens) return launch_wt<kEpiSwiGLU>(g_wt_tokens, A, B, a, lda, ldb, s);
             return g_on_pairs == 3 ? launch_pair_swapped<kEpiSwiGLU>(A, B, a, lda, ldb, s)
                    : g_on_pairs == 2 ? launch_pair_wide<kEpiSwiGLU>(A, B, a, lda, ldb, s)
                    : g_on_pairs ? launch_pair_grouped<kEpiSwiGLU>(A, B, a, lda, ldb, s) : launch<kEpiSwiGLU>(A, B, a, lda, ldb, s);
@@ -575,6 +640,7 @@ static int grouped_gemm_impl(const void* A, const void* B, void* C, const int* g
             for (int i = 0; i < 8; ++i) a.scatter_base[i] = scatter_bases8[i];
             a.scatter_row_bytes = scatter_row_bytes;
             a.scatter_slots     = scatter_slots;
+            if (g_wt_tokens) return launch_wt<kEpiScatterRows>(g_wt_tokens, A, B, a, lda, ldb, s);
             return g_on_pairs == 3 ? launch_pair_swapped<kEpiScatterRows>(A, B, a, lda, ldb, s)
                    : g_on_pairs == 2 ? launch_pair_wide<kEpiScatterRows>(A, B, a, lda, ldb, s)
                    : g_on_pairs ? launch_pair_grouped<kEpiScatterRows>(A, B, a, lda, ldb, s)

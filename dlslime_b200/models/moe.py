@@ -88,11 +88,12 @@ class ExpertParallelMoE:
         # words of the gated GEMM's dynamic tile scheduler (SLIME_EP_STATIC_TILES=1: every gridDim-th tile instead)
         self._tile_counter = None if os.environ.get("SLIME_EP_STATIC_TILES") == "1" else torch.zeros(2, dtype=torch.int32, device=dev)
         # pair_gemm: the expert GEMMs on CTA pairs (True: 256 x 256 tiles, "wide": 256 x 512). They win where a local
-        # expert sees several hundred rows per step (many ranks), and lose to the single-CTA kernel's 128-row tiles on
-        # small groups; SLIME_EP_PAIR_GEMM=0|1|wide overrides the rule, autotune() measures.
+        # expert sees a thousand rows per step (many ranks) and their larger tiles waste little: steps run back to back at the
+        # power limit take 2815 us against 2860 on single CTAs with 32 x 1024 rows, but 3775 against 3300 with 64 x 512 and 3085 against
+        # 2744 with 64 x 384; SLIME_EP_PAIR_GEMM=0|1|wide overrides the rule, autotune() measures.
         rows_per_expert = max_tokens * cfg.topk * self.world // max(1, cfg.num_experts)
         forced = os.environ.get("SLIME_EP_PAIR_GEMM")
-        self.pair_gemm = (rows_per_expert >= 512) if forced is None else {"0": False, "1": True}.get(forced, forced)
+        self.pair_gemm = (rows_per_expert >= 1024) if forced is None else {"0": False, "1": True}.get(forced, forced)
         # tile width of the single-CTA expert GEMMs (0 = 256). Narrower tiles were measured for the decode-size step on
         # many ranks (32 experts x 32 rows: 512 tiles = 3.46 waves of the grid) and do not pay: those GEMMs stream weights
         # from HBM, the CTAs do not wait for one another between waves, and a short last wave still fills the memory
@@ -103,6 +104,11 @@ class ExpertParallelMoE:
         expected = max_tokens * cfg.topk * self.world / max(1, cfg.num_experts)
         forced_m = os.environ.get("SLIME_EP_TILE_M")
         self.tile_m = (64 if expected + 3 * expected ** 0.5 <= 64 else 0) if forced_m is None else int(forced_m)
+        # weights on the M side, a group's rows on the N side (SLIME_EP_TILE_TOKENS=0|64|128|192); autotune's other kinds and the
+        # tile overrides above take precedence
+        forced_t = os.environ.get("SLIME_EP_TILE_TOKENS")
+        free = not self.tile_n_gate_up and forced_m is None
+        self.tile_tokens = int(forced_t) if forced_t is not None else gemm.pick_tile_tokens(expected) if free else 0
         cap = self.buf.recv_cap
         self.xd = torch.empty((cap, cfg.hidden), dtype=torch.bfloat16, device=dev)
         self.h = torch.empty((cap, cfg.intermediate), dtype=torch.bfloat16, device=dev)
@@ -126,20 +132,25 @@ class ExpertParallelMoE:
             self.buf.wait(0, epoch)
         self.buf.recv_dequant(self.xd, epoch, expected_rows=rows)
 
-    def step_gate_up(self):
+    def _tiles(self, tile_n: int, chained: int) -> dict:
+        if self.tile_tokens and not self.pair_gemm:
+            return {"tile_tokens": self.tile_tokens, "chained": chained}
+        return {"pair": self.pair_gemm, "tile_n": tile_n, "tile_m": self.tile_m}
+
+    def step_gate_up(self, chained: int = 0):
         if self.fuse_dequant:
             gemm.grouped_gemm_fp8a(self.buf.recv_x, self.buf.recv_scale, self.w_gate_up, self.buf.group_offsets, out=self.h,
                                    epilogue=gemm.EPI_SWIGLU)
             return
         gemm.grouped_gemm_bf16(self.xd, self.w_gate_up, self.buf.group_offsets, out=self.h, epilogue=gemm.EPI_SWIGLU,
-                               pair=self.pair_gemm, tile_n=self.tile_n_gate_up, tile_m=self.tile_m)
+                               **self._tiles(self.tile_n_gate_up, chained))
 
-    def step_down(self):
+    def step_down(self, chained: int = 0):
         c = self.cfg
         gemm.grouped_gemm_bf16(self.h, self.w_down, self.buf.group_offsets, epilogue=gemm.EPI_SCATTER_ROWS,
                                row_info=self.buf.recv_info, scatter_bases=self._bases,
-                               scatter_row_bytes=c.hidden * 2, scatter_slots=self.max_tokens * c.topk, pair=self.pair_gemm,
-                               tile_n=self.tile_n_down, tile_m=self.tile_m)
+                               scatter_row_bytes=c.hidden * 2, scatter_slots=self.max_tokens * c.topk,
+                               **self._tiles(self.tile_n_down, chained))
 
     def step_experts(self, T, epoch):
         self.step_recv(T, epoch)

@@ -12,6 +12,7 @@ from .. import _lib
 from ._common import default_status, ptr, require_cuda, stream_ptr
 
 EPI_STORE, EPI_SWIGLU, EPI_SCATTER_ROWS = 0, 1, 2
+WT_MAX_ROWS = 224  # see pick_tile_tokens
 
 
 def _wide_tiles_pay(m: int, n: int, sms: int = 148) -> bool:
@@ -79,11 +80,23 @@ def pick_grouped_tile_n(row_tiles: int, n_out: int, swiglu: bool = False, sms: i
     return best
 
 
+def pick_tile_tokens(rows_per_group: float) -> int:
+    """``tile_tokens`` of :func:`grouped_gemm_bf16` for groups that are expected to hold ``rows_per_group`` rows each (0 = the
+    row-tiled forms are the faster ones): the smallest tile that holds a group three standard deviations above the mean, so
+    that a group's weights enter an SM once, and the most stages for it (64 experts x 97 rows: 1082 us a step with tiles of
+    128, 1380 with 64, 1105 with 192). From ``WT_MAX_ROWS`` rows on, between 192 (3321 us against 3541 for the row tiles, 128
+    experts) and 256 (4952 against 4126), the row tiles win."""
+    most = rows_per_group + 3 * rows_per_group ** 0.5
+    if rows_per_group >= WT_MAX_ROWS:
+        return 0
+    return 64 if most <= 64 else 128 if most <= 128 else 192
+
+
 def grouped_gemm_bf16(a: torch.Tensor, b: torch.Tensor, group_offsets: torch.Tensor, out: torch.Tensor | None = None,
                       epilogue: int = EPI_STORE, row_info: torch.Tensor | None = None, scatter_bases=None,
                       scatter_row_bytes: int = 0, scatter_slots: int = 0,
                       row_scale: torch.Tensor | None = None, pair: bool | str = False, tile_n: int = 0,
-                      w_prefetch: int = 0, tile_m: int = 0) -> torch.Tensor | None:
+                      w_prefetch: int = 0, tile_m: int = 0, tile_tokens: int = 0, chained: int = 0) -> torch.Tensor | None:
     """Grouped GEMM over consecutive row groups of ``a``.
 
     ``a`` is ``[M_cap, K]``; ``group_offsets`` is an int32 device tensor of
@@ -105,7 +118,11 @@ def grouped_gemm_bf16(a: torch.Tensor, b: torch.Tensor, group_offsets: torch.Ten
     the weight boxes this many 64-deep K blocks ahead of its loads, meant for launches that stream weights from HBM (few rows per
     group); measured slower than no prefetch at every distance on this part, so nothing sets it. ``tile_m=64`` (single CTAs, 256-wide
     tiles): row tiles of 64 instead of 128, for groups of a few dozen rows (a decode step): the A part of a pipeline stage
-    halves and the ring gets a fifth stage, so more weight bytes are in flight per SM.
+    halves and the ring gets a fifth stage, so more weight bytes are in flight per SM. ``tile_tokens`` (64, 128 or 192; excludes
+    the other tile options): weights on the M side of the MMA, all rows of a group (cut into equal parts above ``tile_tokens``)
+    on the N side: the form for launches that stream weights, see :func:`pick_tile_tokens`. ``chained`` (with ``tile_tokens``):
+    the launch is scheduled while the kernel in front of it in the stream drains; 2 = ``group_offsets`` and ``b`` were
+    complete before that kernel began, so the first weights are fetched without waiting for it.
     """
     require_cuda(a, b, group_offsets)
     assert a.dtype == b.dtype == torch.bfloat16 and group_offsets.dtype == torch.int32
@@ -120,6 +137,12 @@ def grouped_gemm_bf16(a: torch.Tensor, b: torch.Tensor, group_offsets: torch.Ten
     if not pair and (tile_n not in (0, 256) or w_prefetch or tile_m == 64):
         _lib.call("slime_grouped_gemm_bf16_tile", ptr(a), ptr(b), ptr(out), ptr(group_offsets), g, m_cap, n, k, a.stride(0), k, ldc,
                   epilogue, ptr(row_info), scatter_bases, scatter_row_bytes, scatter_slots, ptr(row_scale), int(tile_n), int(w_prefetch), int(tile_m),
+                  default_status().dev_ptr, stream_ptr())
+        return out
+    if tile_tokens:
+        assert not pair and tile_n in (0, 256) and not w_prefetch and tile_m in (0, 128)
+        _lib.call("slime_grouped_gemm_bf16_wt", ptr(a), ptr(b), ptr(out), ptr(group_offsets), g, m_cap, n, k, a.stride(0), k, ldc,
+                  epilogue, ptr(row_info), scatter_bases, scatter_row_bytes, scatter_slots, ptr(row_scale), int(tile_tokens), int(chained),
                   default_status().dev_ptr, stream_ptr())
         return out
     entry = "slime_grouped_gemm_bf16_swapped" if pair == "swap" else "slime_grouped_gemm_bf16_wide" if pair == "wide" else "slime_grouped_gemm_bf16_pair" if pair else "slime_grouped_gemm_bf16"

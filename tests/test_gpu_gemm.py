@@ -214,3 +214,48 @@ def test_grouped_gemm_with_fp8_activations_is_bit_identical_to_dequant_then_gemm
         default_status().check()
         assert torch.equal(out[:total], ref[:total]), (out[:total].float() - ref[:total].float()).abs().max().item()
         assert bool((out[total:] == 0).all())
+
+
+@pytest.mark.parametrize("tile_tokens", [64, 128, 192])
+@pytest.mark.parametrize("sizes,n,k", [([3, 0, 130, 257, 64], 448, 384), ([1], 32, 64), ([16, 17, 128, 129, 192, 193, 385], 288, 1096), ([0, 0, 5], 1024, 512)])
+def test_grouped_gemm_weights_on_the_m_side(sizes, n, k, tile_tokens):
+    """Groups below, at and above one tile of tokens, empty ones, feature tiles that reach past N (into the next group and past the
+    end), a K that is no multiple of 64; store, SwiGLU and scatter with row weights and dropped rows against the fp32 product."""
+    import ctypes
+
+    from dlslime_b200.ops import gemm
+    from dlslime_b200.ops._common import default_status
+
+    torch.manual_seed(n + k + tile_tokens)
+    g, total = len(sizes), sum(sizes)
+    offs = torch.tensor([0] + list(torch.tensor(sizes).cumsum(0)), dtype=torch.int32, device="cuda")
+    a = torch.randn(total + 3, k, device="cuda", dtype=torch.bfloat16)  # rows behind the last group are nobody's
+    w = (torch.randn(g, n, k, device="cuda") * 0.05).to(torch.bfloat16)
+    w2 = (torch.randn(g, 2 * n, k, device="cuda") * 0.05).to(torch.bfloat16)
+    out = torch.full((total + 3, n), 9.0, device="cuda", dtype=torch.bfloat16)
+    gemm.grouped_gemm_bf16(a, w, offs, out=out, tile_tokens=tile_tokens)
+    h = gemm.grouped_gemm_bf16(a, w2, offs, epilogue=gemm.EPI_SWIGLU, tile_tokens=tile_tokens)
+    dst = torch.zeros(total, n, device="cuda", dtype=torch.bfloat16)
+    perm = torch.randperm(total, device="cuda")
+    info = torch.cat([perm, torch.zeros(3, dtype=torch.int64, device="cuda")])
+    info[total // 2] = 5 << 48  # a region that does not exist: the row is dropped
+    scale = torch.rand(total + 3, device="cuda")
+    bases = (ctypes.c_ulonglong * 8)()
+    bases[0] = dst.data_ptr()
+    gemm.grouped_gemm_bf16(a, w, offs, epilogue=gemm.EPI_SCATTER_ROWS, row_info=info, row_scale=scale, scatter_bases=bases,
+                           scatter_row_bytes=n * 2, scatter_slots=total, tile_tokens=tile_tokens)
+    torch.cuda.synchronize()
+    default_status().check()
+    assert (out[total:] == 9.0).all() and (dst[perm[total // 2]] == 0).all()
+    start = 0
+    for gi, sz in enumerate(sizes):
+        rows = slice(start, start + sz)
+        if sz:
+            x = a[rows].float()
+            ref = x @ w[gi].float().t()
+            keep = torch.arange(start, start + sz, device="cuda") != total // 2
+            _check(out[rows], ref, k)
+            if keep.any():
+                _check(dst[perm[rows]][keep], (ref * scale[rows, None])[keep], k)
+            _check(h[rows], torch.nn.functional.silu(x @ w2[gi, :n].float().t()) * (x @ w2[gi, n:].float().t()), k)
+        start += sz
