@@ -116,6 +116,8 @@ __global__ void __launch_bounds__(256) ep_route_kernel(EpConfig cfg, const float
     const int t    = blockIdx.x * 8 + warp;
     const int E    = cfg.num_experts;
     const int K    = cfg.topk;
+    griddep_wait();  // one-rank steps chain their kernels (see launch_chained); a no-op otherwise
+    griddep_launch_dependents();
     epoch          = resolve_epoch(cfg, epoch);  // read by every CTA before it reports in below
     if (t < T) {
         int   my_e = -1;
@@ -262,6 +264,8 @@ __global__ void __launch_bounds__(256) ep_dispatch_kernel(EpConfig cfg, const __
     const int E = cfg.num_experts, El = cfg.experts_per_rank, W = cfg.world, K = cfg.topk, H = cfg.hidden;
     const unsigned long long lim = cfg.wait_ns ? cfg.wait_ns : kDefaultWaitNs;
 
+    griddep_wait();
+    griddep_launch_dependents();
     epoch = resolve_epoch(cfg, epoch);
     if (threadIdx.x == 0) s_ok = 1;
     const unsigned long long trace_t0 = tracing(cfg) ? globaltimer_ns() : 0;
@@ -785,6 +789,8 @@ __global__ void __launch_bounds__(256) ep_combine_reduce_kernel(EpConfig cfg, in
                                                                __nv_bfloat16* __restrict__ out, long long ldo,
                                                                unsigned long long epoch, int do_signal, KernelStatus* st)
 {
+    griddep_wait();
+    griddep_launch_dependents();
     epoch = resolve_epoch(cfg, epoch);
     if (do_signal && blockIdx.x == 0 && threadIdx.x < cfg.world) {
         fence_acq_rel_sys();
@@ -864,6 +870,18 @@ int check_cfg(const EpConfig& c)
     return 0;
 }
 
+// Launches one kernel of a step. With one rank nothing in the step waits for a peer, so the kernels are chained as
+// programmatic dependents: each one's blocks are scheduled while the kernel in front of it drains, and wait for its
+// completion first thing. With more ranks a block that only waits could hold a slot that a peer's progress needs.
+// Three tokens on 32 experts, launched eagerly: 344 -> 336 us a step; no difference where the GEMMs take milliseconds.
+template<typename... KArgs, typename... Args>
+cudaError_t launch_chained(const EpConfig& cfg, void (*kernel)(KArgs...), int grid, cudaStream_t stream, Args&&... args)
+{
+    if (cfg.world == 1) return launch_programmatic(kernel, dim3(grid), dim3(256), 0, stream, static_cast<Args&&>(args)...);
+    kernel<<<grid, 256, 0, stream>>>(static_cast<KArgs>(args)...);
+    return cudaGetLastError();
+}
+
 int grid_for(long long warp_units, int cap_blocks)
 {
     long long blocks = (warp_units + 7) / 8;
@@ -890,10 +908,8 @@ static int route_impl(const void* cfg_bytes, const float* logits, int T, int* to
     if (check_cfg(cfg)) return -1;
     if (T < 0 || T > cfg.max_tokens) return fail("ep route: T=%d exceeds max_tokens=%d", T, cfg.max_tokens);
     const int blocks = T > 0 ? (T + 7) / 8 : 1;
-    ep_route_kernel<<<blocks, 256, 0, static_cast<cudaStream_t>(stream)>>>(cfg, logits, T, topk_idx, topk_w, slot,
-                                                                          send_count, block_counter, epoch, renormalize,
-                                                                          push_off);
-    SLIME_CUDA_OK(cudaGetLastError());
+    SLIME_CUDA_OK(launch_chained(cfg, ep_route_kernel, blocks, static_cast<cudaStream_t>(stream), cfg, logits, T, topk_idx, topk_w, slot,
+                                 send_count, block_counter, epoch, renormalize, push_off));
     return 0;
 }
 
@@ -994,10 +1010,9 @@ static int dispatch_impl(const void* cfg_bytes, const void* x, long long ldx, in
     if (ldx % 8 != 0) return fail("ep dispatch: ldx must be a multiple of 8 elements");
     const long long units = static_cast<long long>(T) * (cfg.hidden / kChunk);
     const int       grid  = grid_for(units, max_blocks > 0 ? max_blocks : sm_count() * 4);
-    ep_dispatch_kernel<kExpand><<<grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(
-        cfg, static_cast<const __nv_bfloat16*>(x), ldx, T, topk_idx, slot, group_offsets, block_counter,
-        static_cast<__nv_bfloat16*>(y), ldy, epoch, static_cast<KernelStatus*>(status));
-    SLIME_CUDA_OK(cudaGetLastError());
+    SLIME_CUDA_OK(launch_chained(cfg, ep_dispatch_kernel<kExpand>, grid, static_cast<cudaStream_t>(stream), cfg,
+                                 static_cast<const __nv_bfloat16*>(x), ldx, T, topk_idx, slot, group_offsets, block_counter,
+                                 static_cast<__nv_bfloat16*>(y), ldy, epoch, static_cast<KernelStatus*>(status)));
     return 0;
 }
 
@@ -1082,10 +1097,8 @@ int slime_ep_combine_reduce(const void* cfg_bytes, int T, const int* topk_idx, c
     if (T < 0 || T > cfg.max_tokens) return fail("ep combine: T=%d exceeds max_tokens=%d", T, cfg.max_tokens);
     const long long units = static_cast<long long>(T) * (cfg.hidden / 256);
     const int       grid  = grid_for(units, sm_count() * 4);
-    ep_combine_reduce_kernel<<<grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(
-        cfg, T, topk_idx, topk_w, static_cast<__nv_bfloat16*>(out), ldo, epoch, do_signal,
-        static_cast<KernelStatus*>(status));
-    SLIME_CUDA_OK(cudaGetLastError());
+    SLIME_CUDA_OK(launch_chained(cfg, ep_combine_reduce_kernel, grid, static_cast<cudaStream_t>(stream), cfg, T, topk_idx, topk_w,
+                                 static_cast<__nv_bfloat16*>(out), ldo, epoch, do_signal, static_cast<KernelStatus*>(status)));
     return 0;
 }
 

@@ -274,8 +274,8 @@ class ExpertParallelMoE:
         if self.world == 1 and not self.fuse_dequant and not self.thin_waits and self.buf.trace is None:
             # one rank: no row crosses a wire, so dispatch writes what the receive would (the trace counts both kernels)
             self.buf.dispatch_expand(x, self.xd, None)
-            self.step_gate_up()
-            self.step_down()
+            self.step_gate_up(chained=1)
+            self.step_down(chained=2)  # the row groups are dispatch's, two kernels back
         else:
             self.step_dispatch(x, None)
             self.step_experts(T, None)
