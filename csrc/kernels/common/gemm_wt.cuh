@@ -166,7 +166,7 @@ gemm_bf16_wt_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_consta
 
     if (warp == 0) {
         // ------------------------------ TMA producer ------------------------------
-        if (lane == 0) {
+        {
             WtWalker<PTOK> walk(args, offs, kFeatOut);
             WtTile   tc;
             int      stage = 0;
@@ -182,25 +182,28 @@ gemm_bf16_wt_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_consta
                 tma_load_2d(sw + S::kWBytes / 2, &tmW, &full_bar[s], kb * kBK, y + (EPI == kEpiSwiGLU ? args.N : 128));
             };
             if (ahead) {
-                if (have)
-                    for (; early < kStages && early < kblocks; ++early) load_w(early, early);
+                if (have && elect_one())
+                    for (int i = 0; i < kStages && i < kblocks; ++i) load_w(i, i);
+                __syncwarp();
+                early = have ? min(kStages, kblocks) : 0;
                 griddep_wait();
             }
             if (args.chained) fence_proxy_async();  // the tokens were written by the kernel in front of this one
             for (; ok && have; have = walk.next(tc)) {
                 for (int kb = 0; kb < kblocks; ++kb) {
-                    if (!mbar_wait(&empty_bar[stage], phase ^ 1, st, 1, stage, lim)) {
+                    if (!__all_sync(0xffffffffu, mbar_wait(&empty_bar[stage], phase ^ 1, st, 1, stage, lim))) {
                         ok = false;
                         break;
                     }
-                    if (early > 0)
-                        --early;
-                    else
-                        load_w(stage, kb);
-                    uint8_t* sx = smem + stage * S::kStageBytes + S::kWBytes;
-                    int      r  = 0;
-                    for (; r + 32 <= tc.ntok; r += 32) tma_load_2d(sx + r * kBK * 2, &tmX32, &full_bar[stage], kb * kBK, tc.tok0 + r);
-                    if (r < tc.ntok) tma_load_2d(sx + r * kBK * 2, &tmX16, &full_bar[stage], kb * kBK, tc.tok0 + r);
+                    if (elect_one()) {
+                        if (early == 0) load_w(stage, kb);
+                        uint8_t* sx = smem + stage * S::kStageBytes + S::kWBytes;
+                        int      r  = 0;
+                        for (; r + 32 <= tc.ntok; r += 32) tma_load_2d(sx + r * kBK * 2, &tmX32, &full_bar[stage], kb * kBK, tc.tok0 + r);
+                        if (r < tc.ntok) tma_load_2d(sx + r * kBK * 2, &tmX16, &full_bar[stage], kb * kBK, tc.tok0 + r);
+                    }
+                    __syncwarp();
+                    if (early > 0) --early;
                     if (++stage == kStages) {
                         stage = 0;
                         phase ^= 1;
@@ -212,7 +215,7 @@ gemm_bf16_wt_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_consta
     }
     else if (warp == 1) {
         // ------------------------------ MMA issuer --------------------------------
-        if (lane == 0) {
+        {
             WtWalker<PTOK> walk(args, offs, kFeatOut);
             WtTile   tc;
             int      stage = 0, acc = 0;
@@ -221,15 +224,15 @@ gemm_bf16_wt_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_consta
             while (ok && walk.next(tc)) {
                 const bool large = tc.ntok > 128;
                 if (large) acc = 0;
-                ok = mbar_wait(&tempty_bar[acc], acc_phase[acc] ^ 1, st, 2, acc, lim)
-                     && (!large || mbar_wait(&tempty_bar[1], acc_phase[1] ^ 1, st, 2, 1, lim));
+                ok = __all_sync(0xffffffffu, mbar_wait(&tempty_bar[acc], acc_phase[acc] ^ 1, st, 2, acc, lim)
+                                                 && (!large || mbar_wait(&tempty_bar[1], acc_phase[1] ^ 1, st, 2, 1, lim)));
                 if (!ok) break;
                 tc_fence_after_sync();
                 const uint32_t idesc  = make_idesc(kFmtBF16, kFmtBF16, 128, static_cast<uint32_t>(tc.ntok));
                 const uint32_t tmem_d = tmem_base + acc * 256;
                 const uint32_t block1 = large ? 256 : 128;
                 for (int kb = 0; kb < kblocks; ++kb) {
-                    if (!mbar_wait(&full_bar[stage], phase, st, 3, stage, lim)) {
+                    if (!__all_sync(0xffffffffu, mbar_wait(&full_bar[stage], phase, st, 3, stage, lim))) {
                         ok = false;
                         break;
                     }
@@ -238,22 +241,28 @@ gemm_bf16_wt_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_consta
                     const uint64_t d0 = make_kmajor_sw128_desc(sw);
                     const uint64_t d1 = make_kmajor_sw128_desc(sw + S::kWBytes / 2);
                     const uint64_t dx = make_kmajor_sw128_desc(sw + S::kWBytes);
+                    if (elect_one()) {
 #pragma unroll
-                    for (int k = 0; k < kBK / 16; ++k) {
-                        umma_f16(tmem_d, d0 + 2 * k, dx + 2 * k, idesc, (kb | k) != 0);
-                        umma_f16(tmem_d + block1, d1 + 2 * k, dx + 2 * k, idesc, (kb | k) != 0);
+                        for (int k = 0; k < kBK / 16; ++k) {
+                            umma_f16(tmem_d, d0 + 2 * k, dx + 2 * k, idesc, (kb | k) != 0);
+                            umma_f16(tmem_d + block1, d1 + 2 * k, dx + 2 * k, idesc, (kb | k) != 0);
+                        }
+                        umma_commit(&empty_bar[stage]);
                     }
-                    umma_commit(&empty_bar[stage]);
+                    __syncwarp();
                     if (++stage == kStages) {
                         stage = 0;
                         phase ^= 1;
                     }
                 }
                 if (!ok) break;
-                umma_commit(&tfull_bar[acc]);
+                if (elect_one()) {
+                    umma_commit(&tfull_bar[acc]);
+                    if (large) umma_commit(&tfull_bar[1]);
+                }
+                __syncwarp();
                 acc_phase[acc] ^= 1;
                 if (large) {
-                    umma_commit(&tfull_bar[1]);
                     acc_phase[1] ^= 1;
                 }
                 else {
