@@ -10,14 +10,16 @@
 // current 32 are added (64 registers beside the 128 accumulators), a partial is handed back as soon as its last read has
 // landed, and the first read of the next one is issued before the last additions when that partial is ready. That is more
 // than the 168 registers that 12 warps may have at launch: the promotion warpgroups take over what the producer's
-// warpgroup gives back (setmaxnreg). PAIRFIG
+// warpgroup gives back (setmaxnreg). A K block now takes 650 cycles, 512 of them MMA, as long as the clock holds; what is left is the
+// power limit: 8192 x 3584 x 8192 309 -> 283 us, 4096 x 4096 x 7168 148 -> 127-139 us, 8192^3 level at 600-610 us (1.8 PFLOP/s).
 // The tiles left over after the last full round of the grid are cut into 2, 4 or 8 column parts of a pair each.
 //
 // Split along K (128 x 256 tiles, cluster of 2, 4 or 8 CTAs): for products with fewer tiles than half of the SMs. Each CTA of
 // a cluster takes an equal run of K blocks and leaves its sums in its shared memory; then each adds one slice of
 // the columns over the cluster, in the order of K, through distributed shared memory, and stores it. Narrower tiles
 // instead have all CTAs read the same rows of A: 72 x 4096 x 7168 took 27 us on 128 CTAs with tiles of 32 columns, and
-// leaving the promotion out changed nothing. KSPLITFIG
+// leaving the promotion out changed nothing. Of the 14 us that 72 rows take in the kernel, 6 are the K blocks and 8 the exchange of
+// the sums. 72 x 4096 x 7168 38.9 -> 21 us, 33 x 2048 x 8192 41 -> 16.4 us, 500 x 2048 x 7168 39 -> 25-29 us.
 #pragma once
 
 #include "gemm_fp8.cuh"
@@ -38,7 +40,8 @@ constexpr int kF8pMaxParts  = 8;
 constexpr int kF8pABytes    = kBM * kF8BK;
 constexpr int kF8pRingBytes = 6 * (kF8pABytes + kF8BN / 2 * kF8BK);  // stages * stage_bytes is at most this
 constexpr int kF8pBarBytes  = (2 * kF8pMaxStages + 2 * kF8pMaxParts) * 8 + 16;
-constexpr int kF8pSmem      = kF8pRingBytes + kF8pBarBytes + 1024;
+constexpr int kF8pEpiBytes  = kF8pPromoWarps * 32 * kEpiRowPitch;  // results leave through one 128-byte slot per row and warp
+constexpr int kF8pSmem      = kF8pRingBytes + kF8pEpiBytes + kF8pBarBytes + 1024;
 static_assert(kF8pSmem <= kSmemLimit, "shared memory budget");
 
 struct F8PairArgs {
@@ -194,7 +197,8 @@ __device__ __forceinline__ bool f8_accumulate(unsigned long long (&acc)[NCH * 16
 // One tile of the pair kernel by one thread: promotion, then its `cols` columns of its row.
 template<int NCH>
 __device__ __forceinline__ bool f8_pair_tile(const F8PairArgs& f, const F8Tile& tc, F8Parts& pp, uint64_t* pfull_bar, uint32_t pempty,
-                                             uint32_t taddr_lane, int grp, int row, int kblocks, unsigned long long lim)
+                                             uint32_t taddr_lane, int grp, int row, int kblocks, uint8_t* warp_slots,
+                                             unsigned long long lim)
 {
     const bool   valid = row < f.M;
     const int    cols  = tc.width / 2;
@@ -205,20 +209,21 @@ __device__ __forceinline__ bool f8_pair_tile(const F8PairArgs& f, const F8Tile& 
     unsigned long long acc[NCH * 16];
     if (!f8_accumulate<NCH>(acc, pp, tc.parts(), tc.part_stride(), pfull_bar, pempty, taddr_lane + grp * cols, sa_row, sb_row, kblocks, f.status, lim))
         return false;
-    if (valid) {
-        __nv_bfloat16* out  = f.C + static_cast<long long>(row) * f.ldc + col0;
-        int            left = f.N - col0;  // a multiple of 8 (N % 32 == 0)
-        if (left > cols) left = cols;
+    // whole 128-byte lines leave the SM (see epi_store_piece); 64 columns at a time, 32 for the narrow tiles
+    int left = f.N - col0;  // a multiple of 8 (N % 32 == 0)
+    if (left > cols) left = cols;
+    const unsigned long long dst = reinterpret_cast<unsigned long long>(f.C + static_cast<long long>(row) * f.ldc + col0);
 #pragma unroll
-        for (int i = 0; i < NCH * 4; ++i) {
-            if (i * 8 < left) {
-                uint32_t o[4];
+    for (int i = 0; i < NCH; i += 2) {
+        uint32_t o[32];
 #pragma unroll
-                for (int j = 0; j < 4; ++j)
-                    o[j] = pack_bf16(__uint_as_float(static_cast<uint32_t>(acc[4 * i + j])), __uint_as_float(static_cast<uint32_t>(acc[4 * i + j] >> 32)));
-                *reinterpret_cast<uint4*>(out + 8 * i) = make_uint4(o[0], o[1], o[2], o[3]);
-            }
+        for (int j = 0; j < 32; ++j) {
+            const int q = i * 16 + j;
+            o[j]        = q < NCH * 16 ? pack_bf16(__uint_as_float(static_cast<uint32_t>(acc[q < NCH * 16 ? q : 0])),
+                                                   __uint_as_float(static_cast<uint32_t>(acc[q < NCH * 16 ? q : 0] >> 32))) : 0u;
         }
+        epi_store_piece(warp_slots + (threadIdx.x & 31) * kEpiRowPitch, warp_slots, o, dst + static_cast<unsigned long long>(i) * 64, valid,
+                        min(64, left - i * 32), threadIdx.x & 31);
     }
     return true;
 }
@@ -242,7 +247,8 @@ gemm_fp8_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
 
-    uint64_t* full_bar   = reinterpret_cast<uint64_t*>(smem + kF8pRingBytes);  // used in the leader only
+    uint8_t*  epi_smem   = smem + kF8pRingBytes;
+    uint64_t* full_bar   = reinterpret_cast<uint64_t*>(epi_smem + kF8pEpiBytes);  // used in the leader only
     uint64_t* empty_bar  = full_bar + kF8pMaxStages;                           // one set per CTA
     uint64_t* pfull_bar  = empty_bar + kF8pMaxStages;                          // one set per CTA
     uint64_t* pempty_bar = pfull_bar + kF8pMaxParts;                           // used in the leader only
@@ -378,6 +384,7 @@ gemm_fp8_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
         const int      grp    = (warp - kF8pCtlWarps) >> 2;  // which half of the tile's columns
         const uint32_t pempty = mapa_u32(pempty_bar, 0);
         const uint32_t taddr  = tmem_base + (static_cast<uint32_t>(quad * 32) << 16);
+        uint8_t*       warp_slots = epi_smem + (warp - kF8pCtlWarps) * 32 * kEpiRowPitch;
         F8PairWalker   walk(f);
         F8Tile         tc;
         F8Parts        pp;
@@ -388,11 +395,11 @@ gemm_fp8_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
             if (width != 0 && width != tc.width) pp.part = 0;  // as the MMA issuer does
             width = tc.width;
             if (tc.width == 256)
-                ok = f8_pair_tile<4>(f, tc, pp, pfull_bar, pempty, taddr, grp, row, kblocks, lim);
+                ok = f8_pair_tile<4>(f, tc, pp, pfull_bar, pempty, taddr, grp, row, kblocks, warp_slots, lim);
             else if (tc.width == 128)
-                ok = f8_pair_tile<2>(f, tc, pp, pfull_bar, pempty, taddr, grp, row, kblocks, lim);
+                ok = f8_pair_tile<2>(f, tc, pp, pfull_bar, pempty, taddr, grp, row, kblocks, warp_slots, lim);
             else
-                ok = f8_pair_tile<1>(f, tc, pp, pfull_bar, pempty, taddr, grp, row, kblocks, lim);
+                ok = f8_pair_tile<1>(f, tc, pp, pfull_bar, pempty, taddr, grp, row, kblocks, warp_slots, lim);
         }
         if (!ok) *fail_slot = 1;
     }
@@ -432,7 +439,7 @@ gemm_fp8_ksplit_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
 
-    uint64_t* full_bar   = reinterpret_cast<uint64_t*>(smem + kF8pRingBytes);
+    uint64_t* full_bar   = reinterpret_cast<uint64_t*>(smem + kF8pRingBytes + kF8pEpiBytes);
     uint64_t* empty_bar  = full_bar + kF8pMaxStages;
     uint64_t* pfull_bar  = empty_bar + kF8pMaxStages;
     uint64_t* pempty_bar = pfull_bar + kF8pMaxParts;

@@ -5,6 +5,7 @@
 // HBM bandwidth: 16-byte loads, 8-byte fp8 stores, amax by shuffles, one multiply per element.
 #include "common/fp8.cuh"
 #include "common/host_utils.h"
+#include "common/ptx.cuh"
 #include "slime_cuda.h"
 
 using namespace slime;
@@ -41,6 +42,7 @@ __global__ void __launch_bounds__(256) quant_1x128_kernel(const __nv_bfloat16* _
                                                          float* __restrict__ scales, long long n_groups,
                                                          int groups_per_row, long long ldx, long long ldq)
 {
+    griddep_launch_dependents();  // a product that reads the result may be scheduled while this kernel drains
     const long long warp = (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
     const int       quad = (threadIdx.x >> 3) & 3, sub = threadIdx.x & 7;
     long long       gid[kQuantPasses], ox[kQuantPasses], oq[kQuantPasses];

@@ -1,6 +1,6 @@
 // Entry points of the block-scaled fp8 GEMM (common/gemm_fp8.cuh): the plain product and the
 // all-gather -> GEMM built on it (fp8 payload and scales cross NVLink, half the bytes of the bf16 form).
-#include "common/gemm_fp8.cuh"
+#include "common/gemm_fp8_pair.cuh"
 #include "common/host_utils.h"
 #include "slime_cuda.h"
 
@@ -50,6 +50,101 @@ int launch_f8(const void* Aq, const void* Bq, const void* A_local, const F8Args&
     return 0;
 }
 
+// Clusters of `size` CTAs of the split kernel that fit on the device at the same time.
+int ksplit_clusters(int size)
+{
+    constexpr int kMaxDev = 64;
+    static int    cached[kMaxDev][4] = {};
+    int           dev = 0;
+    cudaGetDevice(&dev);
+    const int slot = size == 2 ? 0 : size == 4 ? 1 : 2;
+    if (dev >= 0 && dev < kMaxDev && cached[dev][slot]) return cached[dev][slot] - 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim          = dim3(size);
+    cfg.blockDim         = dim3(kF8pThreads);
+    cfg.dynamicSmemBytes = kF8pSmem;
+    cudaLaunchAttribute attr[1];
+    attr[0].id               = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = size;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs                = attr;
+    cfg.numAttrs             = 1;
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, gemm_fp8_ksplit_kernel, &cfg) != cudaSuccess) {
+        cudaGetLastError();
+        n = 0;
+    }
+    if (dev >= 0 && dev < kMaxDev) cached[dev][slot] = n + 1;
+    return n;
+}
+
+// Which form a plain product takes. Fewer 128 x 256 tiles than half of the SMs: one cluster per tile, split along K over as
+// many CTAs as still run at the same time, if that shortens each CTA's run by 14 blocks: meeting twice and adding the sums
+// costs about 6 us (2000 x 544 x 1024: 20.5 us in clusters, 14.3 without). Else, with more than one row tile, CTA pairs: the r tiles that are left over after
+// the last full round are cut into the most column parts (2, 4 or 8) that still have a pair each, since a last round of few
+// wide tiles would take as long as a full one. The rest (one row tile, very wide) stays on single CTAs,
+// and so do all-gathered operands, whose order and pace are set by the arriving shards.
+int launch_plain_f8(const void* Aq, const void* Bq, const F8Args& g, long long lda, long long ldb, cudaStream_t stream)
+{
+    static bool configured = false;
+    if (!configured) {
+        SLIME_CUDA_OK(cudaFuncSetAttribute(gemm_fp8_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kF8pSmem));
+        SLIME_CUDA_OK(cudaFuncSetAttribute(gemm_fp8_ksplit_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kF8pSmem));
+        configured = true;
+    }
+    F8PairArgs f{};
+    f.M = g.M, f.N = g.N, f.K = g.K, f.C = g.C, f.ldc = g.ldc, f.sa = g.sa, f.sb = g.sb, f.status = g.ag.status, f.wait_ns = g.ag.wait_ns;
+    const int  sms     = sm_count();
+    const long ntiles  = (f.N + kF8BN - 1) / kF8BN;
+    const long tiles   = static_cast<long>((f.M + kBM - 1) / kBM) * ntiles;
+    const int  kblocks = f.K / kF8BK;
+    CUtensorMap tmA, tmB, tmBn;
+    if (make_tmap_2d(&tmA, Aq, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, f.M, f.K, lda, kBM, kF8BK)) return -1;
+    if (make_tmap_2d(&tmB, Bq, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, f.N, f.K, ldb, kF8BN / 2, kF8BK)) return -1;
+    int split = 1;
+    if (2 * tiles <= sms)
+        for (int c : {2, 4, 8})
+            if (kblocks - kblocks / c >= 14 && tiles <= ksplit_clusters(c)) split = c;
+    cudaLaunchConfig_t cfg{};
+    cfg.blockDim         = dim3(kF8pThreads);
+    cfg.dynamicSmemBytes = kF8pSmem;
+    cfg.stream           = stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id                                         = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs                                          = attr;
+    cfg.numAttrs                                       = 1;
+    if (split > 1) {
+        f.split                  = split;
+        cfg.gridDim              = dim3(static_cast<unsigned>(tiles * split));
+        attr[1].id               = cudaLaunchAttributeClusterDimension;
+        attr[1].val.clusterDim.x = split;
+        attr[1].val.clusterDim.y = 1;
+        attr[1].val.clusterDim.z = 1;
+        cfg.numAttrs             = 2;
+        SLIME_CUDA_OK(cudaLaunchKernelEx(&cfg, gemm_fp8_ksplit_kernel, tmA, tmB, f));
+        return 0;
+    }
+    if (f.M <= kBM) return launch_f8<false>(Aq, Bq, nullptr, g, lda, ldb, stream);
+    const int  pairs      = sms / 2;
+    const long pair_tiles = static_cast<long>((f.M + 2 * kBM - 1) / (2 * kBM)) * ntiles;
+    const long rest       = pair_tiles % pairs;
+    f.full_tiles          = static_cast<int>(pair_tiles);
+    f.split               = 1;
+    while (f.split < 8 && rest > 0 && rest * f.split * 2 <= pairs) f.split *= 2;
+    if (f.split > 1) f.full_tiles = static_cast<int>(pair_tiles - rest);
+    const int widest = f.full_tiles > 0 ? kF8BN : kF8BN / f.split;
+    f.stage_bytes    = kF8pABytes + widest / 2 * kF8BK;
+    f.stages         = kF8pRingBytes / f.stage_bytes < kF8pMaxStages ? kF8pRingBytes / f.stage_bytes : kF8pMaxStages;
+    tmBn             = tmB;
+    if (f.split > 1 && make_tmap_2d(&tmBn, Bq, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, f.N, f.K, ldb, kF8pNarrowBox, kF8BK)) return -1;
+    const long units = f.full_tiles + (pair_tiles - f.full_tiles) * f.split;
+    cfg.gridDim      = dim3(static_cast<unsigned>(2 * (units < pairs ? units : pairs)));
+    SLIME_CUDA_OK(cudaLaunchKernelEx(&cfg, gemm_fp8_pair_kernel, tmA, tmB, tmBn, f));
+    return 0;
+}
+
 int check_f8(int M, int N, int K, long long lda, long long ldb, long long ldc)
 {
     if (M <= 0 || N <= 0 || K <= 0) return fail("fp8 gemm: M, N, K must be positive (got %d, %d, %d)", M, N, K);
@@ -77,7 +172,7 @@ int slime_gemm_fp8_blockscaled(const void* Aq, const float* sa, const void* Bq, 
     f.sa = sa;
     f.sb = sb;
     f.ag.status = static_cast<KernelStatus*>(status);
-    return launch_f8<false>(Aq, Bq, nullptr, f, lda, ldb, static_cast<cudaStream_t>(stream));
+    return launch_plain_f8(Aq, Bq, f, lda, ldb, static_cast<cudaStream_t>(stream));
 }
 
 // All-gather -> GEMM in fp8. xq_local / sx_local: this rank's quantised shard [rows_local, K] and its scales

@@ -259,3 +259,28 @@ def test_grouped_gemm_weights_on_the_m_side(sizes, n, k, tile_tokens):
                 _check(dst[perm[rows]][keep], (ref * scale[rows, None])[keep], k)
             _check(h[rows], torch.nn.functional.silu(x @ w2[gi, :n].float().t()) * (x @ w2[gi, n:].float().t()), k)
         start += sz
+
+
+@pytest.mark.parametrize("m,n,k", [(1, 32, 128), (72, 4096, 7168), (72, 4096, 1024), (129, 2080, 384), (2400, 2048, 640), (3300, 2048, 256),
+                                   (65, 8192, 1152), (300, 4128, 4096), (257, 288, 2304), (20000, 512, 512)])
+def test_gemm_fp8_forms(m, n, k):
+    """Single CTAs (one block of K), clusters of 2, 4 and 8 that share K unevenly, and CTA pairs with the last round cut into
+    column parts (wide and narrow tiles in one launch, parts past the end of N, rows past M in one CTA of the pair)."""
+    from dlslime_b200.ops import gemm, quant
+    from dlslime_b200.ops._common import default_status
+
+    torch.manual_seed(m + 5 * n + k)
+    a = (torch.randn(m, k, device="cuda") * (torch.rand(m, 1, device="cuda") + 0.1) * 4).to(torch.bfloat16)
+    w = (torch.randn(n, k, device="cuda") * 0.05).to(torch.bfloat16)
+    aq, sa = quant.fp8_quant_1x128(a)
+    wq, sb = quant.fp8_quant_128x128(w)
+    out = torch.full((m + 1, n), 7.0, device="cuda", dtype=torch.bfloat16)
+    gemm.gemm_fp8_blockscaled(aq, sa, wq, sb, out=out[:m])
+    torch.cuda.synchronize()
+    default_status().check()
+    blocks = sb.double().repeat_interleave(128, 0)[:n].repeat_interleave(128, 1)[:, :k]
+    ref = (aq.double() * sa.double().repeat_interleave(128, 1)) @ (wq.double() * blocks).t()
+    # bf16 rounding of the result (2^-9), and k fp32 additions of terms whose magnitudes sum to at most ~sqrt(k) results
+    tol = ref.abs() * 2 ** -8 + ref.pow(2).mean().sqrt() * k ** 0.5 * 2 ** -20
+    assert ((out[:m].double() - ref).abs() <= tol).all()
+    assert (out[m] == 7.0).all(), "a row past the end was written"
