@@ -217,8 +217,9 @@ struct TileFeed {
             phase ^= 1;
         }
     }
-    // Consumer side: the next tile index, -1 at the end (or when the wait ran out, with ok = false).
-    __device__ int take(KernelStatus* st, unsigned long long lim, bool& ok)
+    // Consumer side: the next tile index, -1 at the end (or when the wait ran out, with ok = false). `whole_warp`: all lanes
+    // call this together and count as one consumer.
+    __device__ int take(KernelStatus* st, unsigned long long lim, bool& ok, bool whole_warp = false)
     {
         if (!dynamic) {
             const int t = t_static;
@@ -230,7 +231,8 @@ struct TileFeed {
             return -1;
         }
         const int t = ring[slot];
-        mbar_arrive(&empty[slot]);
+        if (whole_warp) __syncwarp();
+        if (!whole_warp || (threadIdx.x & 31) == 0) mbar_arrive(&empty[slot]);
         advance();
         return t;
     }
@@ -619,7 +621,7 @@ gemm_bf16_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
     }
     else if (warp == 1) {
         // ------------------------------ MMA issuer --------------------------------
-        if (lane == 0) {
+        {  // the whole warp walks, one elected thread issues (see elect_one)
             TileWalker walk(args, kBNOut, AROWS);
             TileCoord  tc;
             int        stage = 0;
@@ -630,16 +632,20 @@ gemm_bf16_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
             constexpr uint32_t idesc = make_idesc(kFmtBF16, kFmtBF16, kBM, BN);
             TileFeed           feed(args, tile_ring, tr_full, tr_empty);
             while (ok) {
-                const int lt = feed.take(st, lim, ok);
+                const int lt = feed.take(st, lim, ok, true);
+                if (!__all_sync(0xffffffffu, ok)) {
+                    ok = false;
+                    break;
+                }
                 if (lt < 0 || !walk.at(lt, tc)) break;
-                if (!mbar_wait(&tempty_bar[acc], acc_phase ^ 1, st, 2, acc, lim)) {
+                if (!__all_sync(0xffffffffu, mbar_wait(&tempty_bar[acc], acc_phase ^ 1, st, 2, acc, lim))) {
                     ok = false;
                     break;
                 }
                 tc_fence_after_sync();
                 const uint32_t tmem_d = tmem_base + acc * kAccStride;
                 for (int kb = 0; kb < kblocks; ++kb) {
-                    if (!mbar_wait(&full_bar[stage], phase, st, 3, stage, lim)) {
+                    if (!__all_sync(0xffffffffu, mbar_wait(&full_bar[stage], phase, st, 3, stage, lim))) {
                         ok = false;
                         break;
                     }
@@ -648,19 +654,23 @@ gemm_bf16_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
                     const uint32_t sb = sa + S::kABytes;
                     const uint64_t da = make_kmajor_sw128_desc(sa);
                     const uint64_t db = make_kmajor_sw128_desc(sb);
+                    if (elect_one()) {
 #pragma unroll
-                    for (int k = 0; k < kBK / 16; ++k) {
-                        // advance 16 bf16 = 32 bytes along K inside the swizzle row: +2 in the >>4 address field
-                        umma_f16(tmem_d, da + 2 * k, db + 2 * k, idesc, (kb | k) != 0);
+                        for (int k = 0; k < kBK / 16; ++k) {
+                            // advance 16 bf16 = 32 bytes along K inside the swizzle row: +2 in the >>4 address field
+                            umma_f16(tmem_d, da + 2 * k, db + 2 * k, idesc, (kb | k) != 0);
+                        }
+                        umma_commit(&empty_bar[stage]);  // frees the smem slot when these MMAs retire
                     }
-                    umma_commit(&empty_bar[stage]);  // frees the smem slot when these MMAs retire
+                    __syncwarp();
                     if (++stage == STAGES) {
                         stage = 0;
                         phase ^= 1;
                     }
                 }
                 if (!ok) break;
-                umma_commit(&tfull_bar[acc]);
+                if (elect_one()) umma_commit(&tfull_bar[acc]);
+                __syncwarp();
                 if (++acc == 2) {
                     acc = 0;
                     acc_phase ^= 1;

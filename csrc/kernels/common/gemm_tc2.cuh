@@ -149,7 +149,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
 
     if (warp == 0) {
         // ------------------------------ TMA producer (both CTAs) ------------------------------
-        if (lane == 0) {
+        {
             PairWalker walk(args, BN, cluster, n_clusters);
             PairTile   tc;
             int        stage = 0;
@@ -167,22 +167,25 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
                 }
                 if (gate) {
                     const int f = my_row0 / args.a_ready_rows;  // a_ready_rows == 128: one counter per CTA half
-                    ok = wait_flag_ge(args.a_ready + f, args.a_ready_target, st, 10, f, lim);
+                    ok = __all_sync(0xffffffffu, wait_flag_ge(args.a_ready + f, args.a_ready_target, st, 10, f, lim));
                     if (!ok) break;
                     fence_proxy_async();
                 }
                 const int yb = tc.nt * BN + static_cast<int>(crank) * (BN / 2);
                 for (int kb = 0; kb < kblocks; ++kb) {
-                    if (!mbar_wait(&empty_bar[stage], phase ^ 1, st, 1, stage, lim)) {
+                    if (!__all_sync(0xffffffffu, mbar_wait(&empty_bar[stage], phase ^ 1, st, 1, stage, lim))) {
                         ok = false;
                         break;
                     }
                     uint8_t* sa = smem + stage * S::kStageBytes;
                     uint8_t* sb = sa + S::kABytes;
-                    if (crank == 0) mbar_arrive_expect_tx(&full_bar[stage], 2 * S::kStageBytes);
-                    const uint32_t leader_full = mapa_u32(&full_bar[stage], 0);
-                    tma_load_2d_pair(sa, mapA, leader_full, kb * kBK, arow);
-                    tma_load_2d_pair(sb, &tmB, leader_full, kb * kBK, yb);
+                    if (elect_one()) {
+                        if (crank == 0) mbar_arrive_expect_tx(&full_bar[stage], 2 * S::kStageBytes);
+                        const uint32_t leader_full = mapa_u32(&full_bar[stage], 0);
+                        tma_load_2d_pair(sa, mapA, leader_full, kb * kBK, arow);
+                        tma_load_2d_pair(sb, &tmB, leader_full, kb * kBK, yb);
+                    }
+                    __syncwarp();
                     if (++stage == STAGES) {
                         stage = 0;
                         phase ^= 1;
@@ -194,7 +197,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
     }
     else if (warp == 1) {
         // ------------------------------ MMA issuer (leader only) ------------------------------
-        if (lane == 0 && crank == 0) {
+        if (crank == 0) {  // the whole warp walks, one elected thread issues
             PairWalker walk(args, BN, cluster, n_clusters);
             PairTile   tc;
             int        stage = 0;
@@ -204,14 +207,14 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
             bool       ok = true;
             constexpr uint32_t idesc = make_idesc(kFmtBF16, kFmtBF16, kPairBM, BN);
             while (ok && walk.next(tc)) {
-                if (!mbar_wait(&tempty_bar[acc], acc_phase ^ 1, st, 2, acc, lim)) {
+                if (!__all_sync(0xffffffffu, mbar_wait(&tempty_bar[acc], acc_phase ^ 1, st, 2, acc, lim))) {
                     ok = false;
                     break;
                 }
                 tc_fence_after_sync();
                 const uint32_t tmem_d = tmem_base + acc * kAccStride;
                 for (int kb = 0; kb < kblocks; ++kb) {
-                    if (!mbar_wait(&full_bar[stage], phase, st, 3, stage, lim)) {
+                    if (!__all_sync(0xffffffffu, mbar_wait(&full_bar[stage], phase, st, 3, stage, lim))) {
                         ok = false;
                         break;
                     }
@@ -220,16 +223,20 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
                     const uint32_t sb = sa + S::kABytes;
                     const uint64_t da = make_kmajor_sw128_desc(sa);
                     const uint64_t db = make_kmajor_sw128_desc(sb);
+                    if (elect_one()) {
 #pragma unroll
-                    for (int k = 0; k < kBK / 16; ++k) umma_f16_pair(tmem_d, da + 2 * k, db + 2 * k, idesc, (kb | k) != 0);
-                    umma_commit_pair(&empty_bar[stage], 3);  // frees the stage in both CTAs
+                        for (int k = 0; k < kBK / 16; ++k) umma_f16_pair(tmem_d, da + 2 * k, db + 2 * k, idesc, (kb | k) != 0);
+                        umma_commit_pair(&empty_bar[stage], 3);  // frees the stage in both CTAs
+                    }
+                    __syncwarp();
                     if (++stage == STAGES) {
                         stage = 0;
                         phase ^= 1;
                     }
                 }
                 if (!ok) break;
-                umma_commit_pair(&tfull_bar[acc], 3);  // the accumulator halves of both CTAs are complete
+                if (elect_one()) umma_commit_pair(&tfull_bar[acc], 3);  // the accumulator halves of both CTAs are complete
+                __syncwarp();
                 if (++acc == 2) {
                     acc = 0;
                     acc_phase ^= 1;

@@ -164,7 +164,7 @@ gemm_bf16_pair_swapped_kernel(const __grid_constant__ CUtensorMap tmW, const __g
 
     if (warp == 0) {
         // ------------------------------ TMA producer (both CTAs) ------------------------------
-        if (lane == 0) {
+        {
             SwapWalker walk(args, kFeatOut, cluster, n_clusters);
             SwapTile   tc;
             int        stage = 0;
@@ -176,22 +176,25 @@ gemm_bf16_pair_swapped_kernel(const __grid_constant__ CUtensorMap tmW, const __g
                 // this CTA's half of the tile's tokens
                 const int xrow = tc.tok0 + static_cast<int>(crank) * (tc.ntok / 2);
                 for (int kb = 0; kb < kblocks; ++kb) {
-                    if (!mbar_wait(&empty_bar[stage], phase ^ 1, st, 1, stage, lim)) {
+                    if (!__all_sync(0xffffffffu, mbar_wait(&empty_bar[stage], phase ^ 1, st, 1, stage, lim))) {
                         ok = false;
                         break;
                     }
                     uint8_t* sw = smem + stage * S::kStageBytes;
                     uint8_t* sx = sw + S::kWBytes;
-                    if (crank == 0) mbar_arrive_expect_tx(&full_bar[stage], 2 * S::kStageBytes);
-                    const uint32_t leader_full = mapa_u32(&full_bar[stage], 0);
-                    if (EPI == kEpiSwiGLU) {  // the weight map's box is 64 rows
-                        tma_load_2d_pair(sw, &tmW, leader_full, kb * kBK, wrow);
-                        tma_load_2d_pair(sw + S::kWBytes / 2, &tmW, leader_full, kb * kBK, wrow + args.N);
+                    if (elect_one()) {
+                        if (crank == 0) mbar_arrive_expect_tx(&full_bar[stage], 2 * S::kStageBytes);
+                        const uint32_t leader_full = mapa_u32(&full_bar[stage], 0);
+                        if (EPI == kEpiSwiGLU) {  // the weight map's box is 64 rows
+                            tma_load_2d_pair(sw, &tmW, leader_full, kb * kBK, wrow);
+                            tma_load_2d_pair(sw + S::kWBytes / 2, &tmW, leader_full, kb * kBK, wrow + args.N);
+                        }
+                        else {
+                            tma_load_2d_pair(sw, &tmW, leader_full, kb * kBK, wrow);
+                        }
+                        tma_load_2d_pair(sx, &tmX, leader_full, kb * kBK, xrow);
                     }
-                    else {
-                        tma_load_2d_pair(sw, &tmW, leader_full, kb * kBK, wrow);
-                    }
-                    tma_load_2d_pair(sx, &tmX, leader_full, kb * kBK, xrow);
+                    __syncwarp();
                     if (++stage == STAGES) {
                         stage = 0;
                         phase ^= 1;
@@ -203,7 +206,7 @@ gemm_bf16_pair_swapped_kernel(const __grid_constant__ CUtensorMap tmW, const __g
     }
     else if (warp == 1) {
         // ------------------------------ MMA issuer (leader only) ------------------------------
-        if (lane == 0 && crank == 0) {
+        if (crank == 0) {  // the whole warp walks, one elected thread issues
             SwapWalker walk(args, kFeatOut, cluster, n_clusters);
             SwapTile   tc;
             int        stage = 0;
@@ -212,7 +215,7 @@ gemm_bf16_pair_swapped_kernel(const __grid_constant__ CUtensorMap tmW, const __g
             uint32_t   acc_phase = 0;
             bool       ok = true;
             while (ok && walk.next(tc)) {
-                if (!mbar_wait(&tempty_bar[acc], acc_phase ^ 1, st, 2, acc, lim)) {
+                if (!__all_sync(0xffffffffu, mbar_wait(&tempty_bar[acc], acc_phase ^ 1, st, 2, acc, lim))) {
                     ok = false;
                     break;
                 }
@@ -220,7 +223,7 @@ gemm_bf16_pair_swapped_kernel(const __grid_constant__ CUtensorMap tmW, const __g
                 const uint32_t idesc  = make_idesc(kFmtBF16, kFmtBF16, kPairBM, static_cast<uint32_t>(tc.ntok));
                 const uint32_t tmem_d = tmem_base + acc * kAccStride;
                 for (int kb = 0; kb < kblocks; ++kb) {
-                    if (!mbar_wait(&full_bar[stage], phase, st, 3, stage, lim)) {
+                    if (!__all_sync(0xffffffffu, mbar_wait(&full_bar[stage], phase, st, 3, stage, lim))) {
                         ok = false;
                         break;
                     }
@@ -228,16 +231,20 @@ gemm_bf16_pair_swapped_kernel(const __grid_constant__ CUtensorMap tmW, const __g
                     const uint32_t sw = smem_u32(smem + stage * S::kStageBytes);
                     const uint64_t da = make_kmajor_sw128_desc(sw);                // weights: the M operand
                     const uint64_t db = make_kmajor_sw128_desc(sw + S::kWBytes);   // tokens: the N operand
+                    if (elect_one()) {
 #pragma unroll
-                    for (int k = 0; k < kBK / 16; ++k) umma_f16_pair(tmem_d, da + 2 * k, db + 2 * k, idesc, (kb | k) != 0);
-                    umma_commit_pair(&empty_bar[stage], 3);  // frees the stage in both CTAs
+                        for (int k = 0; k < kBK / 16; ++k) umma_f16_pair(tmem_d, da + 2 * k, db + 2 * k, idesc, (kb | k) != 0);
+                        umma_commit_pair(&empty_bar[stage], 3);  // frees the stage in both CTAs
+                    }
+                    __syncwarp();
                     if (++stage == STAGES) {
                         stage = 0;
                         phase ^= 1;
                     }
                 }
                 if (!ok) break;
-                umma_commit_pair(&tfull_bar[acc], 3);  // the accumulator halves of both CTAs are complete
+                if (elect_one()) umma_commit_pair(&tfull_bar[acc], 3);  // the accumulator halves of both CTAs are complete
+                __syncwarp();
                 if (++acc == 2) {
                     acc = 0;
                     acc_phase ^= 1;

@@ -167,7 +167,7 @@ gemm_bf16_pair_wide_kernel(const __grid_constant__ CUtensorMap tmA, const __grid
 
     if (warp == 0) {
         // ------------------------------ TMA producer (both CTAs) ------------------------------
-        if (lane == 0) {
+        {
             WideWalker walk(args, kTileOut, cluster, n_clusters);
             WideTile   tc;
             int        stage = 0;
@@ -184,17 +184,20 @@ gemm_bf16_pair_wide_kernel(const __grid_constant__ CUtensorMap tmA, const __grid
                         yb[j] = tc.group * args.rowsB + tc.nt * kTileOut + j * BN + static_cast<int>(crank) * (BN / 2);
                 }
                 for (int kb = 0; kb < kblocks; ++kb) {
-                    if (!mbar_wait(&empty_bar[stage], phase ^ 1, st, 1, stage, lim)) {
+                    if (!__all_sync(0xffffffffu, mbar_wait(&empty_bar[stage], phase ^ 1, st, 1, stage, lim))) {
                         ok = false;
                         break;
                     }
                     uint8_t* sa = smem + stage * S::kStageBytes;
                     uint8_t* sb = sa + S::kABytes;
-                    if (crank == 0) mbar_arrive_expect_tx(&full_bar[stage], 2 * S::kStageBytes);
-                    const uint32_t leader_full = mapa_u32(&full_bar[stage], 0);
-                    tma_load_2d_pair(sa, &tmA, leader_full, kb * kBK, arow);
-                    tma_load_2d_pair(sb, &tmB, leader_full, kb * kBK, yb[0]);
-                    tma_load_2d_pair(sb + S::kBHalfBytes, &tmB, leader_full, kb * kBK, yb[1]);
+                    if (elect_one()) {
+                        if (crank == 0) mbar_arrive_expect_tx(&full_bar[stage], 2 * S::kStageBytes);
+                        const uint32_t leader_full = mapa_u32(&full_bar[stage], 0);
+                        tma_load_2d_pair(sa, &tmA, leader_full, kb * kBK, arow);
+                        tma_load_2d_pair(sb, &tmB, leader_full, kb * kBK, yb[0]);
+                        tma_load_2d_pair(sb + S::kBHalfBytes, &tmB, leader_full, kb * kBK, yb[1]);
+                    }
+                    __syncwarp();
                     if (++stage == STAGES) {
                         stage = 0;
                         phase ^= 1;
@@ -206,7 +209,7 @@ gemm_bf16_pair_wide_kernel(const __grid_constant__ CUtensorMap tmA, const __grid
     }
     else if (warp == 1) {
         // ------------------------------ MMA issuer (leader only) ------------------------------
-        if (lane == 0 && crank == 0) {
+        if (crank == 0) {  // the whole warp walks, one elected thread issues
             WideWalker walk(args, kTileOut, cluster, n_clusters);
             WideTile   tc;
             int        stage = 0;
@@ -217,7 +220,7 @@ gemm_bf16_pair_wide_kernel(const __grid_constant__ CUtensorMap tmA, const __grid
             while (ok && walk.next(tc)) {
                 const bool two = tc.nt * kTileOut + kBNOut < args.N;  // block 1 holds columns of the output
                 for (int kb = 0; kb < kblocks && ok; ++kb) {
-                    if (!mbar_wait(&full_bar[stage], phase, st, 3, stage, lim)) {
+                    if (!__all_sync(0xffffffffu, mbar_wait(&full_bar[stage], phase, st, 3, stage, lim))) {
                         ok = false;
                         break;
                     }
@@ -227,7 +230,7 @@ gemm_bf16_pair_wide_kernel(const __grid_constant__ CUtensorMap tmA, const __grid
 #pragma unroll
                     for (int j = 0; j < 2; ++j) {
                         if (kb == 0) {  // the epilogue has drained this block of the previous tile
-                            if (!mbar_wait(&tempty_bar[j], tile_phase ^ 1, st, 2, j, lim)) {
+                            if (!__all_sync(0xffffffffu, mbar_wait(&tempty_bar[j], tile_phase ^ 1, st, 2, j, lim))) {
                                 ok = false;
                                 break;
                             }
@@ -235,21 +238,29 @@ gemm_bf16_pair_wide_kernel(const __grid_constant__ CUtensorMap tmA, const __grid
                         }
                         if (j == 0 || two) {
                             const uint64_t db = make_kmajor_sw128_desc(sa + S::kABytes + j * S::kBHalfBytes);
+                            if (elect_one()) {
 #pragma unroll
-                            for (int k = 0; k < kBK / 16; ++k)
-                                umma_f16_pair(tmem_base + j * kAccStride, da + 2 * k, db + 2 * k, idesc, (kb | k) != 0);
+                                for (int k = 0; k < kBK / 16; ++k)
+                                    umma_f16_pair(tmem_base + j * kAccStride, da + 2 * k, db + 2 * k, idesc, (kb | k) != 0);
+                            }
+                            __syncwarp();
                         }
-                        if (kb == kblocks - 1 && j == 0) umma_commit_pair(&tfull_bar[0], 3);  // block 0 is complete
+                        if (kb == kblocks - 1 && j == 0) {  // block 0 is complete
+                            if (elect_one()) umma_commit_pair(&tfull_bar[0], 3);
+                            __syncwarp();
+                        }
                     }
                     if (!ok) break;
-                    umma_commit_pair(&empty_bar[stage], 3);  // frees the stage in both CTAs
+                    if (elect_one()) umma_commit_pair(&empty_bar[stage], 3);  // frees the stage in both CTAs
+                    __syncwarp();
                     if (++stage == STAGES) {
                         stage = 0;
                         phase ^= 1;
                     }
                 }
                 if (!ok) break;
-                umma_commit_pair(&tfull_bar[1], 3);
+                if (elect_one()) umma_commit_pair(&tfull_bar[1], 3);
+                __syncwarp();
                 tile_phase ^= 1;
             }
             if (!ok) *fail_slot = 1;
