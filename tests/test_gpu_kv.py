@@ -83,7 +83,8 @@ def test_prefill_sender_pushes_every_layer_with_flags():
         assert torch.equal(got[:, :, b, :n], sender.kv_stage[:, :, t:t + n])
 
 
-@pytest.mark.parametrize("page,row,lens,threads", [(1, 8, [5, 1], 256), (7, 2056, [7, 20, 1], 256), (16, 128, [1000, 16, 3], 32), (64, 512, [63, 65, 640], 96)])
+@pytest.mark.parametrize("page,row,lens,threads", [(1, 8, [5, 1], 256), (7, 2056, [7, 20, 1], 256), (16, 128, [1000, 16, 3], 32), (64, 512, [63, 65, 640], 96), (64, 512, [63, 65, 640], 256),
+                                                   (40, 1000, [41] * 40, 256)])
 def test_page_sizes_that_are_no_multiple_of_a_slice(page, row, lens, threads):
     """Pages below, above and beside the 4 KB slices that a warp moves, from a page of 16 bytes on; short last pages, CTAs of
     one, three and eight warps, fewer CTAs than slices; nothing outside the pages' rows is written."""
