@@ -90,10 +90,12 @@ class ExpertParallelMoE:
         # pair_gemm: the expert GEMMs on CTA pairs (True: 256 x 256 tiles, "wide": 256 x 512). They win where a local
         # expert sees a thousand rows per step (many ranks) and their larger tiles waste little: steps run back to back at the
         # power limit take 2815 us against 2860 on single CTAs with 32 x 1024 rows, but 3775 against 3300 with 64 x 512 and 3085 against
-        # 2744 with 64 x 384; SLIME_EP_PAIR_GEMM=0|1|wide overrides the rule, autotune() measures.
+        # 2744 with 64 x 384. "swap" (weights on the M side of a pair) wins between 176 and 320 rows, see gemm.pick_tile_tokens;
+        # SLIME_EP_PAIR_GEMM=0|1|wide|swap overrides the rule, autotune() measures.
         rows_per_expert = max_tokens * cfg.topk * self.world // max(1, cfg.num_experts)
         forced = os.environ.get("SLIME_EP_PAIR_GEMM")
-        self.pair_gemm = (rows_per_expert >= 1024) if forced is None else {"0": False, "1": True}.get(forced, forced)
+        swap = gemm.WT_MAX_ROWS <= rows_per_expert < gemm.SWAP_MAX_ROWS
+        self.pair_gemm = (rows_per_expert >= 1024 or (swap and "swap")) if forced is None else {"0": False, "1": True}.get(forced, forced)
         # tile width of the single-CTA expert GEMMs (0 = 256). Narrower tiles were measured for the decode-size step on
         # many ranks (32 experts x 32 rows: 512 tiles = 3.46 waves of the grid) and do not pay: those GEMMs stream weights
         # from HBM, the CTAs do not wait for one another between waves, and a short last wave still fills the memory

@@ -12,7 +12,7 @@ from .. import _lib
 from ._common import default_status, ptr, require_cuda, stream_ptr
 
 EPI_STORE, EPI_SWIGLU, EPI_SCATTER_ROWS = 0, 1, 2
-WT_MAX_ROWS = 224  # see pick_tile_tokens
+WT_MAX_ROWS, SWAP_MAX_ROWS = 176, 320  # rows per group up to which tile_tokens and pair="swap" are the faster forms
 
 
 def _wide_tiles_pay(m: int, n: int, sms: int = 148) -> bool:
@@ -84,8 +84,10 @@ def pick_tile_tokens(rows_per_group: float) -> int:
     """``tile_tokens`` of :func:`grouped_gemm_bf16` for groups that are expected to hold ``rows_per_group`` rows each (0 = the
     row-tiled forms are the faster ones): the smallest tile that holds a group three standard deviations above the mean, so
     that a group's weights enter an SM once, and the most stages for it (64 experts x 97 rows: 1082 us a step with tiles of
-    128, 1380 with 64, 1105 with 192). From ``WT_MAX_ROWS`` rows on, between 192 (3321 us against 3541 for the row tiles, 128
-    experts) and 256 (4952 against 4126), the row tiles win."""
+    128, 1380 with 64, 1105 with 192). Between ``WT_MAX_ROWS``
+    and ``SWAP_MAX_ROWS`` rows the swapped pairs win, whose tiles hold 256 (128 experts: 160 rows 2430 us here, 2450 on swapped pairs,
+    3080 with row tiles; 192 rows 2950, 2640, 3140; 256 rows 4210, 3555, 3745), from there on the row tiles (64 experts x 384 rows:
+    2552-2612 us on swapped pairs, 2600 with row tiles; 512 rows 3310, 3200)."""
     most = rows_per_group + 3 * rows_per_group ** 0.5
     if rows_per_group >= WT_MAX_ROWS:
         return 0
