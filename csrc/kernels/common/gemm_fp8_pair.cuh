@@ -14,7 +14,7 @@
 // power limit: 8192 x 3584 x 8192 309 -> 283 us, 4096 x 4096 x 7168 148 -> 127-139 us, 8192^3 level at 600-610 us (1.8 PFLOP/s).
 // The tiles left over after the last full round of the grid are cut into 2, 4 or 8 column parts of a pair each.
 //
-// Split along K (128 x 256 tiles, cluster of 2, 4 or 8 CTAs): for products with fewer tiles than half of the SMs. Each CTA of
+// Split along K (128 x 256 tiles, cluster of 2, 4 or 8 CTAs): for products with fewer tiles than a quarter of the SMs. Each CTA of
 // a cluster takes an equal run of K blocks and leaves its sums in its shared memory; then each adds one slice of
 // the columns over the cluster, in the order of K, through distributed shared memory, and stores it. Narrower tiles
 // instead have all CTAs read the same rows of A: 72 x 4096 x 7168 took 27 us on 128 CTAs with tiles of 32 columns, and
@@ -417,13 +417,6 @@ gemm_fp8_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
         tc_fence_after_sync();
         tmem_dealloc_pair(tmem_base, 512);
     }
-}
-
-__device__ __forceinline__ float4 ld_cluster_f32x4(uint32_t cluster_addr)
-{
-    float4 v;
-    asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(cluster_addr) : "memory");
-    return v;
 }
 
 constexpr int kF8kStages     = 4;

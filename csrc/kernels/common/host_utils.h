@@ -109,6 +109,35 @@ inline cudaError_t launch_programmatic(void (*kernel)(KArgs...), dim3 grid, dim3
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
 }
 
+// Clusters of `size` (2, 4 or 8) CTAs of `kernel` that fit on the current device at the same time, kept per device ordinal
+// in `cached`; the kernel's shared-memory attribute has been set.
+template<typename K>
+inline int max_active_clusters(K kernel, int size, int threads, int smem, int (&cached)[64][3])
+{
+    int       dev  = 0;
+    const int slot = size == 2 ? 0 : size == 4 ? 1 : 2;
+    if (cudaGetDevice(&dev) != cudaSuccess) return 0;
+    if (dev >= 0 && dev < 64 && cached[dev][slot]) return cached[dev][slot] - 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim          = dim3(size);
+    cfg.blockDim         = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cudaLaunchAttribute attr[1];
+    attr[0].id               = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = size;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs                = attr;
+    cfg.numAttrs             = 1;
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess) {
+        cudaGetLastError();
+        n = 0;
+    }
+    if (dev >= 0 && dev < 64) cached[dev][slot] = n + 1;
+    return n;
+}
+
 // Multiprocessor count of the current device (cached per device ordinal: a process may drive several GPUs).
 inline int sm_count()
 {

@@ -4,6 +4,7 @@
 // weighted rows to arbitrary (possibly peer) addresses.
 #include "common/gemm_tc2s.cuh"
 #include "common/gemm_tc2w.cuh"
+#include "common/gemm_ks.cuh"
 #include "common/gemm_wt.cuh"
 #include "common/host_utils.h"
 #include "slime_cuda.h"
@@ -74,6 +75,50 @@ int launch_bn(const void* A, const void* B, const void* A_local, int rows_local,
 thread_local int g_tile_n     = 0;  // set around one grouped launch on single CTAs: tile width 128 / 192 / 224 (0 = 256)
 thread_local int g_w_prefetch = 0;  // and the distance of its weight prefetch in K blocks (0 = none)
 thread_local int g_tile_m     = 0;  // 64: row tiles of 64 with a five-stage ring (groups of a few dozen rows)
+
+// CTAs per tile for a product with fewer 128 x 256 tiles than a quarter of the SMs: as many (2, 4 or 8) as all run at the same
+// time, if that shortens each CTA's run by 14 K blocks, about what meeting twice and adding the sums costs. 1 = no split.
+int pick_ksplit(int M, int N, int K)
+{
+    static int  cached[64][3] = {};
+    static bool configured    = false;
+    const long  tiles   = static_cast<long>((M + kBM - 1) / kBM) * ((N + kKsBN - 1) / kKsBN);
+    const int   kblocks = (K + kBK - 1) / kBK;
+    if (4 * tiles > sm_count()) return 1;
+    if (!configured) {
+        if (cudaFuncSetAttribute(gemm_bf16_ksplit_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kKsSmem) != cudaSuccess) {
+            cudaGetLastError();
+            return 1;
+        }
+        configured = true;
+    }
+    int split = 1;
+    for (int c : {2, 4, 8})
+        if (kblocks - kblocks / c >= 14 && tiles <= max_active_clusters(gemm_bf16_ksplit_kernel, c, kThreads, kKsSmem, cached)) split = c;
+    return split;
+}
+
+int launch_ksplit(const void* A, const void* B, const Args& args, long long lda, long long ldb, int split, cudaStream_t stream)
+{
+    CUtensorMap tmA, tmB;
+    if (make_tmap_2d(&tmA, A, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, args.M_total, args.K, lda, kBM, kBK)) return -1;
+    if (make_tmap_2d(&tmB, B, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, args.N, args.K, ldb, kKsBN / 2, kBK)) return -1;
+    const long tiles = static_cast<long>((args.M_total + kBM - 1) / kBM) * ((args.N + kKsBN - 1) / kKsBN);
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim          = dim3(static_cast<unsigned>(tiles * split));
+    cfg.blockDim         = dim3(kThreads);
+    cfg.dynamicSmemBytes = kKsSmem;
+    cfg.stream           = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id               = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = split;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs                = attr;
+    cfg.numAttrs             = 1;
+    SLIME_CUDA_OK(cudaLaunchKernelEx(&cfg, gemm_bf16_ksplit_kernel, tmA, tmB, args, split));
+    return 0;
+}
 
 template<int EPI>
 int launch(const void* A, const void* B, const Args& args, long long lda, long long ldb, cudaStream_t stream)
@@ -318,6 +363,8 @@ int slime_gemm_bf16(const void* A, const void* B, void* C, int M, int N, int K, 
     a.C          = static_cast<__nv_bfloat16*>(C);
     a.ldc        = ldc;
     a.status     = static_cast<KernelStatus*>(status);
+    const int split = pick_ksplit(M, N, K);
+    if (split > 1 && (reinterpret_cast<unsigned long long>(C) & 7) == 0) return launch_ksplit(A, B, a, lda, ldb, split, static_cast<cudaStream_t>(stream));
     return launch<kEpiStore>(A, B, a, lda, ldb, static_cast<cudaStream_t>(stream));
 }
 

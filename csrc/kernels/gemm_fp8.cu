@@ -50,36 +50,13 @@ int launch_f8(const void* Aq, const void* Bq, const void* A_local, const F8Args&
     return 0;
 }
 
-// Clusters of `size` CTAs of the split kernel that fit on the device at the same time.
 int ksplit_clusters(int size)
 {
-    constexpr int kMaxDev = 64;
-    static int    cached[kMaxDev][4] = {};
-    int           dev = 0;
-    cudaGetDevice(&dev);
-    const int slot = size == 2 ? 0 : size == 4 ? 1 : 2;
-    if (dev >= 0 && dev < kMaxDev && cached[dev][slot]) return cached[dev][slot] - 1;
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim          = dim3(size);
-    cfg.blockDim         = dim3(kF8pThreads);
-    cfg.dynamicSmemBytes = kF8pSmem;
-    cudaLaunchAttribute attr[1];
-    attr[0].id               = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = size;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.attrs                = attr;
-    cfg.numAttrs             = 1;
-    int n = 0;
-    if (cudaOccupancyMaxActiveClusters(&n, gemm_fp8_ksplit_kernel, &cfg) != cudaSuccess) {
-        cudaGetLastError();
-        n = 0;
-    }
-    if (dev >= 0 && dev < kMaxDev) cached[dev][slot] = n + 1;
-    return n;
+    static int cached[64][3] = {};
+    return max_active_clusters(gemm_fp8_ksplit_kernel, size, kF8pThreads, kF8pSmem, cached);
 }
 
-// Which form a plain product takes. Fewer 128 x 256 tiles than half of the SMs: one cluster per tile, split along K over as
+// Which form a plain product takes. Fewer 128 x 256 tiles than a quarter of the SMs: one cluster per tile, split along K over as
 // many CTAs as still run at the same time, if that shortens each CTA's run by 14 blocks: meeting twice and adding the sums
 // costs about 6 us (2000 x 544 x 1024: 20.5 us in clusters, 14.3 without). Else, with more than one row tile, CTA pairs: the r tiles that are left over after
 // the last full round are cut into the most column parts (2, 4 or 8) that still have a pair each, since a last round of few
@@ -103,7 +80,7 @@ int launch_plain_f8(const void* Aq, const void* Bq, const F8Args& g, long long l
     if (make_tmap_2d(&tmA, Aq, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, f.M, f.K, lda, kBM, kF8BK)) return -1;
     if (make_tmap_2d(&tmB, Bq, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, f.N, f.K, ldb, kF8BN / 2, kF8BK)) return -1;
     int split = 1;
-    if (2 * tiles <= sms)
+    if (4 * tiles <= sms)
         for (int c : {2, 4, 8})
             if (kblocks - kblocks / c >= 14 && tiles <= ksplit_clusters(c)) split = c;
     cudaLaunchConfig_t cfg{};

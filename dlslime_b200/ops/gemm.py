@@ -47,7 +47,8 @@ def gemm_bf16_pair(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor | None = 
 
 
 def gemm_bf16(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor | None = None, pair: bool | None = None) -> torch.Tensor:
-    """``out[M, N] = a[M, K] @ b[N, K].T``. ``pair`` picks the CTA-pair kernel (default: when M >= 256)."""
+    """``out[M, N] = a[M, K] @ b[N, K].T``. ``pair`` picks the CTA-pair kernel (default: when M >= 256, unless a deep product has
+    so few tiles that clusters which share each tile's K fill the chip better)."""
     require_cuda(a, b)
     assert a.dtype == b.dtype == torch.bfloat16 and a.stride(1) == 1 and b.stride(1) == 1
     m, k = a.shape
@@ -56,7 +57,8 @@ def gemm_bf16(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor | None = None,
     if out is None:
         out = torch.empty((m, n), dtype=torch.bfloat16, device=a.device)
     if pair is None:
-        pair = m >= 256  # two SMs per 256-row tile pay off as soon as there is a full tile
+        few = -(-m // 128) * -(-n // 256) <= 37 and k >= 2048  # four CTAs a tile still fit, and each has eight K blocks
+        pair = m >= 256 and not few  # two SMs per 256-row tile pay off as soon as there is a full tile
     if pair:
         return gemm_bf16_pair(a, b, out)
     _lib.call("slime_gemm_bf16", ptr(a), ptr(b), ptr(out), m, n, k, a.stride(0), b.stride(0), out.stride(0),

@@ -284,3 +284,21 @@ def test_gemm_fp8_forms(m, n, k):
     tol = ref.abs() * 2 ** -8 + ref.pow(2).mean().sqrt() * k ** 0.5 * 2 ** -20
     assert ((out[:m].double() - ref).abs() <= tol).all()
     assert (out[m] == 7.0).all(), "a row past the end was written"
+
+
+@pytest.mark.parametrize("m,n,k", [(1, 32, 2048), (72, 4096, 7168), (129, 544, 4104), (300, 1056, 8192), (500, 2048, 2056), (128, 8192, 1984)])
+def test_gemm_bf16_few_tiles_share_k(m, n, k):
+    """Products with few output tiles: clusters of 2, 4 and 8 CTAs per tile, a K that they share unevenly, rows past M and tile
+    columns past N; rows behind the last one stay."""
+    from dlslime_b200.ops import gemm
+    from dlslime_b200.ops._common import default_status
+
+    torch.manual_seed(m + n + k)
+    a = torch.randn(m, k, device="cuda", dtype=torch.bfloat16)
+    b = (torch.randn(n, k, device="cuda") * 0.05).to(torch.bfloat16)
+    out = torch.full((m + 1, n), 7.0, device="cuda", dtype=torch.bfloat16)
+    gemm.gemm_bf16(a, b, out=out[:m])
+    torch.cuda.synchronize()
+    default_status().check()
+    _check(out[:m], a.float() @ b.float().t(), k)
+    assert (out[m] == 7.0).all()
