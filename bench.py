@@ -474,11 +474,11 @@ def run_ours(args, rank, world, local):
 
     res.update({
         "breakdown_us": dict(breakdown, note="one extra pass with the phases run one after the other, whatever the timed loop does"),
-        "launches": (18 if tbo is not None else 8 if layer.streamed else 6) * args.steps, "cuda_graph": graph is not None, "overlap": tbo is not None,
+        "launches": (18 if tbo is not None else 8 if layer.streamed else 5 if layer.world == 1 and not args.fuse_dequant else 6) * args.steps, "cuda_graph": graph is not None, "overlap": tbo is not None,
         "weights_gb": (layer.w_gate_up.numel() + layer.w_down.numel()) * 2 / 1e9,
-        "notes": {"dequant": "in the gate/up GEMM's A-tile loader" if args.fuse_dequant else "separate pass",
+        "notes": {"dequant": "in the gate/up GEMM's A-tile loader" if args.fuse_dequant else "in dispatch (one rank)" if layer.world == 1 and tbo is None and not layer.streamed else "separate pass",
                   "phases": "dispatch, receive and gate/up GEMM at the same time (per-expert arrival words)" if layer.streamed else "one after the other",
-                  "expert_gemm": {False: "single CTAs, 128 x 256 tiles", True: "CTA pairs, 256 x 256 tiles", "wide": "CTA pairs, 256 x 512 tiles", "swap": "CTA pairs, operands swapped: 256 weight rows x up to 256 tokens"}[layer.pair_gemm],
+                  "expert_gemm": {False: f"single CTAs, 256 weight rows x up to {layer.tile_tokens} tokens" if layer.tile_tokens else "single CTAs, 128 x 256 tiles", True: "CTA pairs, 256 x 256 tiles", "wide": "CTA pairs, 256 x 512 tiles", "swap": "CTA pairs, operands swapped: 256 weight rows x up to 256 tokens"}[layer.pair_gemm],
                   "phases_autotune": tuned,
                   "transport": "in-kernel stores and bulk copies to NVLink peer memory"},
     })
