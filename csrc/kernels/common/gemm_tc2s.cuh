@@ -18,12 +18,11 @@
 // Tiles of a group: ceil(rows / 256) equal parts (rounded up to 16 tokens), part fastest, then the feature tile
 // (256 weight rows per pair: 256 output columns, or 128 for SwiGLU).
 //
-// Measured (32 / 64 / 128 / 256 experts with 1024 / 512 / 256 / 128 rows on average, router-like sizes): level with the
-// 256 x 256 pair kernel at 1024 rows per expert (gate/up 1.373 against 1.368 ms), and behind the single-CTA kernel on
-// smaller groups (256 x 128: 3.34 + 1.80 ms against 2.67 + 1.38 ms) although it computes a third fewer rows and reads
-// the weights from L2 once instead of 1.5 times: those launches stream weights from HBM, and 148 CTAs that each
-// keep 128 KB of weight tiles in flight pull more from HBM than 74 pairs with 96 KB per CTA. The expert-parallel layer
-// times this form with the others (`ExpertParallelMoE.autotune`) and has not picked it so far.
+// Measured as whole one-rank steps (hidden 7168, intermediate 2048), run back to back at the power limit, against row tiles on single
+// CTAs: 128 experts x 192 rows 2640 against 3139 us, x 224 2890 / 3161, x 256 3555 / 3744, 64 x 384 2580 / 2600, x 512 3310 / 3200, 32 x 1024
+// 2870 / 2860. The layer takes it from 176 to 320 rows per expert; below, the tiles of gemm_wt.cuh hold a group as well and need no
+// partner. Loading only the token rows that exist, with boxes of 32 and 8 instead of one of 128, was slower (256 rows: 3850 -> 4209 us):
+// more TMA operations cost more than the bytes they save.
 #pragma once
 
 #include "gemm_tc2g.cuh"

@@ -101,7 +101,7 @@ class ExpertParallelMoE:
         # from HBM, the CTAs do not wait for one another between waves, and a short last wave still fills the memory
         # system (5.66 TB/s of weights with 256-wide tiles, 5.53 with the widths that fill the waves).
         self.tile_n_gate_up = self.tile_n_down = int(os.environ.get("SLIME_EP_TILE_N", "0"))
-        # row tiles of 64 where a local expert is expected to see a few dozen rows per step (decode steps): the A part of
+        # with the tokens on the M side (tile_tokens = 0 below): row tiles of 64 where a local expert is expected to see a few dozen rows per step (decode steps): the A part of
         # a pipeline stage halves, the ring gets a fifth stage and more weight bytes are in flight (SLIME_EP_TILE_M=0|64)
         expected = max_tokens * cfg.topk * self.world / max(1, cfg.num_experts)
         forced_m = os.environ.get("SLIME_EP_TILE_M")
