@@ -109,6 +109,19 @@ inline cudaError_t launch_programmatic(void (*kernel)(KArgs...), dim3 grid, dim3
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
 }
 
+// Dynamic shared memory above the default, once per device (the attribute belongs to the device's copy of the kernel).
+template<typename K>
+inline cudaError_t allow_dynamic_smem(K kernel, int bytes, bool (&done)[64])
+{
+    int         dev = 0;
+    cudaError_t e   = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    if (dev >= 0 && dev < 64 && done[dev]) return cudaSuccess;
+    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    if (e == cudaSuccess && dev >= 0 && dev < 64) done[dev] = true;
+    return e;
+}
+
 // Clusters of `size` (2, 4 or 8) CTAs of `kernel` that fit on the current device at the same time, kept per device ordinal
 // in `cached`; the kernel's shared-memory attribute has been set.
 template<typename K>

@@ -80,17 +80,14 @@ thread_local int g_tile_m     = 0;  // 64: row tiles of 64 with a five-stage rin
 // time, if that shortens each CTA's run by 14 K blocks, about what meeting twice and adding the sums costs. 1 = no split.
 int pick_ksplit(int M, int N, int K)
 {
-    static int  cached[64][3] = {};
-    static bool configured    = false;
+    static int  cached[64][3]  = {};
+    static bool configured[64] = {};
     const long  tiles   = static_cast<long>((M + kBM - 1) / kBM) * ((N + kKsBN - 1) / kKsBN);
     const int   kblocks = (K + kBK - 1) / kBK;
     if (4 * tiles > sm_count()) return 1;
-    if (!configured) {
-        if (cudaFuncSetAttribute(gemm_bf16_ksplit_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kKsSmem) != cudaSuccess) {
-            cudaGetLastError();
-            return 1;
-        }
-        configured = true;
+    if (allow_dynamic_smem(gemm_bf16_ksplit_kernel, kKsSmem, configured) != cudaSuccess) {
+        cudaGetLastError();
+        return 1;
     }
     int split = 1;
     for (int c : {2, 4, 8})
@@ -313,11 +310,8 @@ int launch_wt(const void* A, const void* B, const Args& args, long long lda, lon
     if (make_tmap_2d(&tmX32, A, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, args.M_total, args.K, lda, 32, kBK)) return -1;
     if (make_tmap_2d(&tmX16, A, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, args.M_total, args.K, lda, 16, kBK)) return -1;
     auto kern = gemm_bf16_wt_kernel<PTOK, EPI>;
-    static bool configured = false;
-    if (!configured) {
-        SLIME_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, S::kTotal));
-        configured = true;
-    }
+    static bool configured[64] = {};
+    SLIME_CUDA_OK(allow_dynamic_smem(kern, S::kTotal, configured));
     if (args.chained) {
         SLIME_CUDA_OK(launch_programmatic(kern, dim3(sm_count()), dim3(kWtThreads), S::kTotal, stream, tmW, tmX32, tmX16, args));
         return 0;

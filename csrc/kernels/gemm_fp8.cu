@@ -64,12 +64,9 @@ int ksplit_clusters(int size)
 // and so do all-gathered operands, whose order and pace are set by the arriving shards.
 int launch_plain_f8(const void* Aq, const void* Bq, const F8Args& g, long long lda, long long ldb, cudaStream_t stream)
 {
-    static bool configured = false;
-    if (!configured) {
-        SLIME_CUDA_OK(cudaFuncSetAttribute(gemm_fp8_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kF8pSmem));
-        SLIME_CUDA_OK(cudaFuncSetAttribute(gemm_fp8_ksplit_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kF8pSmem));
-        configured = true;
-    }
+    static bool pairs_configured[64] = {}, clusters_configured[64] = {};
+    SLIME_CUDA_OK(allow_dynamic_smem(gemm_fp8_pair_kernel, kF8pSmem, pairs_configured));
+    SLIME_CUDA_OK(allow_dynamic_smem(gemm_fp8_ksplit_kernel, kF8pSmem, clusters_configured));
     F8PairArgs f{};
     f.M = g.M, f.N = g.N, f.K = g.K, f.C = g.C, f.ldc = g.ldc, f.sa = g.sa, f.sb = g.sb, f.status = g.ag.status, f.wait_ns = g.ag.wait_ns;
     const int  sms     = sm_count();

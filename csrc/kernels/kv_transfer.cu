@@ -298,13 +298,8 @@ int slime_kv_transfer(unsigned long long tok_k, unsigned long long tok_v, unsign
         long long                ctas  = max_blocks > 0 ? max_blocks : sm_count();
         if (ctas > items) ctas = items;
         if (ctas < 1) ctas = 1;
-        static bool configured[64] = {false};
-        int         dev = 0;
-        SLIME_CUDA_OK(cudaGetDevice(&dev));
-        if (dev < 0 || dev >= 64 || !configured[dev]) {
-            SLIME_CUDA_OK(cudaFuncSetAttribute(kv_bulk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kKvRingBytes));
-            if (dev >= 0 && dev < 64) configured[dev] = true;
-        }
+        static bool configured[64] = {};
+        SLIME_CUDA_OK(allow_dynamic_smem(kv_bulk_kernel, kKvRingBytes, configured));
         kv_bulk_kernel<<<static_cast<int>(ctas), 32, kKvRingBytes, static_cast<cudaStream_t>(stream)>>>(a);
         SLIME_CUDA_OK(cudaGetLastError());
         return 0;
