@@ -550,6 +550,7 @@ gemm_fp8_ksplit_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
         }
     }
 
+    __syncwarp();  // the rows past the end of A have split the last warp: an aligned barrier is for whole warps
     cluster_sync_all();  // the sums of all CTAs of the cluster are in place
     {
         // this CTA's slice of the columns, four at a time: N is a multiple of 32, so four columns exist together or not at all

@@ -43,6 +43,20 @@ def test_every_device_wait_goes_through_the_bounded_helpers():
                 assert "globaltimer_ns" in window or "limit" in window, f"{p.name}:{i}: unbounded wait"
 
 
+def test_cluster_barriers_are_reached_by_whole_warps():
+    """barrier.cluster is used in its aligned form, which a split warp must not execute: the statement in front of every one
+    brings the warp (or the block) together."""
+    bad = []
+    for p in KERNELS:
+        prev = ""
+        for i, line in _code_lines(p):
+            if re.search(r"(?<!void )\bcluster_sync_all\(\)", line) and not re.search(r"__sync(threads|warp)\(\);\s*$", prev):
+                bad.append((p.name, i))
+            if line.strip():
+                prev = line.rstrip()
+    assert not bad, bad
+
+
 def test_c_api_header_and_library_agree():
     """Every function declared in the public C headers is exported by the built kernel library."""
     from dlslime_b200 import _lib
