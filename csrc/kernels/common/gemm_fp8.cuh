@@ -408,10 +408,7 @@ gemm_fp8_blockscaled_kernel(const __grid_constant__ CUtensorMap tmA, const __gri
     tc_fence_before_sync();
     __syncthreads();
     if (warp == 1) {
-        if (*fail_slot != 0) {
-            const unsigned long long t0 = globaltimer_ns();
-            while (globaltimer_ns() - t0 < 200000ull) __nanosleep(1000);
-        }
+        if (*fail_slot != 0) settle_copies();
         tc_fence_after_sync();
         tmem_dealloc(tmem_base, kTmemCols);
     }

@@ -410,10 +410,7 @@ gemm_fp8_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
     __syncthreads();
     cluster_sync_all();
     if (warp == 1) {
-        if (*fail_slot != 0) {
-            const unsigned long long t0 = globaltimer_ns();
-            while (globaltimer_ns() - t0 < 200000ull) __nanosleep(1000);
-        }
+        if (*fail_slot != 0) settle_copies();
         tc_fence_after_sync();
         tmem_dealloc_pair(tmem_base, 512);
     }
@@ -577,10 +574,7 @@ gemm_fp8_ksplit_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
     __syncthreads();
     cluster_sync_all();
     if (warp == 1) {
-        if (*fail_slot != 0) {
-            const unsigned long long t0 = globaltimer_ns();
-            while (globaltimer_ns() - t0 < 200000ull) __nanosleep(1000);
-        }
+        if (*fail_slot != 0) settle_copies();
         tc_fence_after_sync();
         tmem_dealloc(tmem_base, 512);
     }

@@ -816,8 +816,7 @@ gemm_bf16_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
     if (warp == 1) {
         if (*fail_slot != 0) {
             // a wait ran out somewhere: give copies still in flight a bounded moment to land
-            const unsigned long long t0 = globaltimer_ns();
-            while (globaltimer_ns() - t0 < 200000ull) __nanosleep(1000);
+            settle_copies();
         }
         tc_fence_after_sync();
         tmem_dealloc(tmem_base, kTmemCols);

@@ -363,10 +363,7 @@ gemm_bf16_pair_wide_kernel(const __grid_constant__ CUtensorMap tmA, const __grid
     __syncthreads();
     cluster_sync_all();
     if (warp == 1) {
-        if (*fail_slot != 0) {
-            const unsigned long long t0 = globaltimer_ns();
-            while (globaltimer_ns() - t0 < 200000ull) __nanosleep(1000);
-        }
+        if (*fail_slot != 0) settle_copies();
         tc_fence_after_sync();
         tmem_dealloc_pair(tmem_base, kTmemCols);
     }

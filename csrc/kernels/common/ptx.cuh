@@ -390,6 +390,13 @@ __device__ __forceinline__ void tma_store_wait()
 {
     asm volatile("cp.async.bulk.wait_group %0;" ::"n"(N) : "memory");
 }
+// For a CTA that leaves because a wait ran out: copies which it has started may still be on their way into its shared
+// memory (and MMAs into its tensor memory), which the next CTA on this SM is going to own. A bounded moment to land.
+__device__ __forceinline__ void settle_copies()
+{
+    const unsigned long long t0 = globaltimer_ns();
+    while (globaltimer_ns() - t0 < 200000ull) __nanosleep(1000);
+}
 // Untiled bulk copy global -> shared (both addresses 16-byte aligned, size a multiple of 16).
 __device__ __forceinline__ void bulk_load_g2s(void* smem_dst, const void* gsrc, uint32_t bytes, uint64_t* bar)
 {

@@ -19,8 +19,8 @@ __global__ void __launch_bounds__(32) ag_push_only_f8_kernel(const F8Args f)
         fence_mbar_init();
     }
     __syncthreads();
-    if (threadIdx.x == 0)
-        ag_push_bulk_f8(f, bufs, bars, 4, blockIdx.x, gridDim.x, f.ag.status, f.ag.wait_ns ? f.ag.wait_ns : kDefaultWaitNs);
+    if (threadIdx.x == 0 && !ag_push_bulk_f8(f, bufs, bars, 4, blockIdx.x, gridDim.x, f.ag.status, f.ag.wait_ns ? f.ag.wait_ns : kDefaultWaitNs))
+        settle_copies();
 }
 
 template<bool AG>

@@ -240,16 +240,18 @@ __global__ void __launch_bounds__(32) kv_bulk_kernel(const __grid_constant__ KvA
     }
     if (lane == 0) {
         while (ok && n_st < n_ld) store_next();
+        if (!ok) settle_copies();
         tma_store_wait<0>();  // every byte has been written before the CTA reports in
         fence_proxy_async();
         if (a.done_flag != nullptr) {
             fence_acq_rel_sys();
-            // a CTA whose wait ran out counts itself in with a mark: then the bytes are not announced
-            constexpr unsigned int kMark = 1u << 24;
-            const unsigned int     old   = atomicAdd(a.block_counter, ok ? 1u : 1u + kMark);
+            // a CTA whose wait ran out leaves a mark before it counts itself in: then the bytes are not announced
+            constexpr unsigned int kMark = 1u << 31;
+            if (!ok) atomicOr(a.block_counter, kMark);
+            const unsigned int old = atomicAdd(a.block_counter, 1u);
             if ((old & (kMark - 1)) == gridDim.x - 1) {
                 fence_acq_rel_sys();
-                if (ok && old < kMark) st_release_sys(a.done_flag, a.done_value);
+                if ((old & kMark) == 0) st_release_sys(a.done_flag, a.done_value);
                 *a.block_counter = 0;
             }
         }

@@ -273,9 +273,9 @@ __global__ void __launch_bounds__(32) p2p_bulk_kernel(const __grid_constant__ Co
                 issue_load();
             }
         }
+        if (!ok) settle_copies();
         tma_store_wait<0>();  // every byte has been written before the CTA reports in
         fence_proxy_async();
-        (void)ok;
         if (a.signal != nullptr) {
             fence_acq_rel_sys();
             if (atomicAdd(a.block_counter, 1u) == gridDim.x - 1) {

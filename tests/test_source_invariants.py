@@ -57,6 +57,19 @@ def test_cluster_barriers_are_reached_by_whole_warps():
     assert not bad, bad
 
 
+def test_kernels_that_load_in_bulk_let_their_copies_land():
+    """A CTA that leaves after a wait ran out must not hand its shared memory on while copies into it are under way: every
+    kernel that starts such copies has the bounded pause of settle_copies() on that path."""
+    loads = re.compile(r"\b(bulk_load_g2s|tma_load_2d\w*|ag_push_bulk\w*)\(")
+    bad = []
+    for p in KERNELS:
+        text = "\n".join(line for _, line in _code_lines(p))
+        for body in text.split("__global__")[1:]:
+            if loads.search(body) and "settle_copies()" not in body:
+                bad.append((p.name, body.split("(", 3)[0].split()[-1], body[:80]))
+    assert not bad, bad
+
+
 def test_c_api_header_and_library_agree():
     """Every function declared in the public C headers is exported by the built kernel library."""
     from dlslime_b200 import _lib
