@@ -350,7 +350,7 @@ gemm_fp8_blockscaled_kernel(const __grid_constant__ CUtensorMap tmA, const __gri
                     // the scales of a gathered shard arrive with its payload: this thread reads them with plain loads,
                     // so it has to see the arrival counter itself (the producer's wait orders only the TMA loads)
                     const int fl = row0 / f.ag.a_ready_rows;
-                    if (!wait_flag_ge(f.ag.a_ready + fl, f.ag.a_ready_target, st, 11, fl, lim)) {
+                    if (!__all_sync(0xffffffffu, wait_flag_ge(f.ag.a_ready + fl, f.ag.a_ready_target, st, 11, fl, lim))) {
                         ok = false;
                         break;
                     }
@@ -366,7 +366,7 @@ gemm_fp8_blockscaled_kernel(const __grid_constant__ CUtensorMap tmA, const __gri
             for (int kb = 0; kb < kblocks; ++kb) {
                 const float s = s_next;
                 if (kb + 1 < kblocks) s_next = sa_row[kb + 1] * sb_row[kb + 1];
-                if (!mbar_wait(&pfull_bar[part], part_phase, st, 4, part, lim)) {
+                if (!mbar_wait_warp(&pfull_bar[part], part_phase, st, 4, part, lim)) {
                     ok = false;
                     break;
                 }

@@ -217,22 +217,22 @@ struct TileFeed {
             phase ^= 1;
         }
     }
-    // Consumer side: the next tile index, -1 at the end (or when the wait ran out, with ok = false). `whole_warp`: all lanes
-    // call this together and count as one consumer.
-    __device__ int take(KernelStatus* st, unsigned long long lim, bool& ok, bool whole_warp = false)
+    // Consumer side, called by all lanes of a warp together: the next tile index, -1 at the end (or when the wait ran out, with
+    // ok = false, in all lanes alike). `one_consumer`: the warp counts as one consumer instead of 32.
+    __device__ int take(KernelStatus* st, unsigned long long lim, bool& ok, bool one_consumer = false)
     {
         if (!dynamic) {
             const int t = t_static;
             t_static += gridDim.x;
             return t;
         }
-        if (!mbar_wait(&full[slot], phase, st, 6, slot, lim)) {
+        if (!mbar_wait_warp(&full[slot], phase, st, 6, slot, lim)) {
             ok = false;
             return -1;
         }
         const int t = ring[slot];
-        if (whole_warp) __syncwarp();
-        if (!whole_warp || (threadIdx.x & 31) == 0) mbar_arrive(&empty[slot]);
+        if (one_consumer) __syncwarp();
+        if (!one_consumer || (threadIdx.x & 31) == 0) mbar_arrive(&empty[slot]);
         advance();
         return t;
     }
@@ -633,10 +633,6 @@ gemm_bf16_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
             TileFeed           feed(args, tile_ring, tr_full, tr_empty);
             while (ok) {
                 const int lt = feed.take(st, lim, ok, true);
-                if (!__all_sync(0xffffffffu, ok)) {
-                    ok = false;
-                    break;
-                }
                 if (lt < 0 || !walk.at(lt, tc)) break;
                 if (!__all_sync(0xffffffffu, mbar_wait(&tempty_bar[acc], acc_phase ^ 1, st, 2, acc, lim))) {
                     ok = false;
@@ -737,7 +733,7 @@ gemm_bf16_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
             const int lt = feed.take(st, lim, feed_ok);
             if (!feed_ok) *fail_slot = 1;
             if (lt < 0 || !walk.at(lt, tc)) break;
-            if (!mbar_wait(&tfull_bar[acc], acc_phase, st, 4, acc, lim)) {
+            if (!mbar_wait_warp(&tfull_bar[acc], acc_phase, st, 4, acc, lim)) {
                 *fail_slot = 1;
                 break;
             }

@@ -260,7 +260,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
         uint32_t       acc_phase = 0;
         const uint32_t leader_tempty[2] = {mapa_u32(&tempty_bar[0], 0), mapa_u32(&tempty_bar[1], 0)};
         while (walk.next(tc)) {
-            if (!mbar_wait(&tfull_bar[acc], acc_phase, st, 4, acc, lim)) {
+            if (!mbar_wait_warp(&tfull_bar[acc], acc_phase, st, 4, acc, lim)) {
                 *fail_slot = 1;
                 break;
             }

@@ -295,7 +295,7 @@ gemm_bf16_pair_wide_kernel(const __grid_constant__ CUtensorMap tmA, const __grid
             else {
                 drow = reinterpret_cast<unsigned long long>(args.C + static_cast<long long>(row) * args.ldc + col0);
             }
-            if (!mbar_wait_relaxed(&tfull_bar[j], tile_phase, st, 4, j, lim)) {
+            if (!mbar_wait_relaxed_warp(&tfull_bar[j], tile_phase, st, 4, j, lim)) {
                 *fail_slot = 1;
                 break;
             }

@@ -348,6 +348,19 @@ __device__ __forceinline__ bool mbar_wait_relaxed(uint64_t* bar, uint32_t parity
     return true;
 }
 
+// The waits for a role that runs as a whole warp: every lane gets the same answer. A limit can run out for one lane and not
+// for another, and what follows (tcgen05.ld, a warp barrier or vote) has to be reached by all lanes or by none.
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, KernelStatus* st, unsigned int where,
+                                               unsigned int aux, unsigned long long limit_ns = kDefaultWaitNs)
+{
+    return __all_sync(0xffffffffu, mbar_wait(bar, parity, st, where, aux, limit_ns));
+}
+__device__ __forceinline__ bool mbar_wait_relaxed_warp(uint64_t* bar, uint32_t parity, KernelStatus* st, unsigned int where,
+                                                       unsigned int aux, unsigned long long limit_ns = kDefaultWaitNs)
+{
+    return __all_sync(0xffffffffu, mbar_wait_relaxed(bar, parity, st, where, aux, limit_ns));
+}
+
 // ---------------------------------------------------------------------------
 // TMA (tiled, 2D). Loads complete on an mbarrier; stores use bulk groups.
 // The x coordinate times the element size must be a multiple of 16 bytes.

@@ -70,6 +70,22 @@ def test_kernels_that_load_in_bulk_let_their_copies_land():
     assert not bad, bad
 
 
+def test_waits_of_whole_warps_end_alike_in_all_lanes():
+    """The roles that read accumulators or take tile numbers run as whole warps. Their bounded waits (places 4 and 6 of the status
+    page, and 11 in the fp8 product) may run out in one lane only, so the lanes vote, or the threads pass the word on before a
+    named barrier."""
+    bad = []
+    for p in KERNELS:
+        lines = [line for _, line in _code_lines(p)]
+        for i, line in enumerate(lines):
+            places = "4|6|11" if p.name == "gemm_fp8.cuh" else "4|6"
+            if re.search(rf"(mbar_wait\w*|wait_flag_ge)\(.*\bst, ({places}),", line):
+                voted = "__all_sync" in line or re.search(r"mbar_wait\w*_warp\(", line)
+                if not voted and not any("epi_fail" in t for t in lines[i: i + 8]):
+                    bad.append((p.name, i + 1))
+    assert not bad, bad
+
+
 def test_c_api_header_and_library_agree():
     """Every function declared in the public C headers is exported by the built kernel library."""
     from dlslime_b200 import _lib
