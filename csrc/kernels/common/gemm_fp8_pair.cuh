@@ -22,6 +22,7 @@
 // the sums. 72 x 4096 x 7168 38.9 -> 21 us, 33 x 2048 x 8192 41 -> 16.4 us, 500 x 2048 x 7168 39 -> 25-29 us.
 #pragma once
 
+#include "cluster_sum.cuh"
 #include "gemm_fp8.cuh"
 
 namespace slime {
@@ -418,8 +419,7 @@ gemm_fp8_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
 
 constexpr int kF8kStages     = 4;
 constexpr int kF8kStageBytes = kBM * kF8BK + kF8BN * kF8BK;
-constexpr int kF8kSumPitch   = kF8BN + 4;  // floats per row of the sums: 16-byte accesses of eight rows hit all banks
-static_assert(kF8kStages * kF8kStageBytes >= kF8kSumPitch * kBM * 4, "the ring holds the sums of the tile afterwards");
+static_assert(kF8BN == kSumCols && kF8kStages * kF8kStageBytes >= kSumPitch * kBM * 4, "the ring holds the sums of the tile afterwards");
 static_assert(kF8kStages * kF8kStageBytes <= kF8pRingBytes, "same shared memory as the pair kernel");
 
 // One 128 x 256 tile per cluster of f.split CTAs, each with its run of K blocks.
@@ -474,7 +474,7 @@ gemm_fp8_ksplit_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
     griddep_wait();
     griddep_launch_dependents();
 
-    float* sums = reinterpret_cast<float*>(smem);  // [128 rows][kF8kSumPitch], once the ring has been consumed
+    float* sums = reinterpret_cast<float*>(smem);  // [128 rows][kSumPitch], once the ring has been consumed
     if (warp < kF8pCtlWarps) {
         setmaxnreg_dec<kF8pRegsCtl>();
         if (warp == 0) {
@@ -536,10 +536,10 @@ gemm_fp8_ksplit_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
         const bool ok = f8_accumulate<4>(acc, pp, 2, kF8BN, pfull_bar, mapa_u32(pempty_bar, static_cast<uint32_t>(crank)),
                                          tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + grp * 128, sa_row, sb_row, kblocks, st, lim);
         if (!ok) *fail_slot = 1;
-        // Every block of this CTA has gone through the tensor core, so the ring is free. (After a wait that ran out a copy
-        // may still land on the sums: the result is void then, and reported.)
-        if (row < f.M) {
-            float4* dst = reinterpret_cast<float4*>(sums + trow * kF8kSumPitch + grp * 128);
+        // Every block of this CTA has gone through the tensor core, so the ring is free. (After a wait that ran out copies may
+        // still land there: nothing is left in it, and nobody stores.)
+        if (ok && row < f.M) {
+            float4* dst = reinterpret_cast<float4*>(sums + trow * kSumPitch + grp * 128);
 #pragma unroll
             for (int i = 0; i < 32; ++i)
                 dst[i] = make_float4(__uint_as_float(static_cast<uint32_t>(acc[2 * i])), __uint_as_float(static_cast<uint32_t>(acc[2 * i] >> 32)),
@@ -547,27 +547,7 @@ gemm_fp8_ksplit_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
         }
     }
 
-    __syncwarp();  // the rows past the end of A have split the last warp: an aligned barrier is for whole warps
-    cluster_sync_all();  // the sums of all CTAs of the cluster are in place
-    {
-        // this CTA's slice of the columns, four at a time: N is a multiple of 32, so four columns exist together or not at all
-        const int quads = kF8BN / f.split / 4;
-        const int rows  = min(kBM, f.M - row0);
-        for (int i = threadIdx.x; i < rows * quads; i += blockDim.x) {
-            const int r = i / quads;
-            const int c = (crank * quads + i % quads) * 4;
-            if (col0 + c >= f.N) continue;
-            float4 v[8];
-#pragma unroll
-            for (int j = 0; j < 8; ++j)
-                if (j < f.split) v[j] = ld_cluster_f32x4(mapa_u32(sums + r * kF8kSumPitch + c, static_cast<uint32_t>(j)));
-            float4 a = v[0];
-#pragma unroll
-            for (int j = 1; j < 8; ++j)
-                if (j < f.split) a = make_float4(a.x + v[j].x, a.y + v[j].y, a.z + v[j].z, a.w + v[j].w);
-            *reinterpret_cast<uint2*>(f.C + static_cast<long long>(row0 + r) * f.ldc + col0 + c) = make_uint2(pack_bf16(a.x, a.y), pack_bf16(a.z, a.w));
-        }
-    }
+    cluster_add_store(sums, fail_slot, crank, f.split, row0, col0, f.M, f.N, f.C, f.ldc);
 
     // teardown: no CTA may leave while another one still reads its sums
     tc_fence_before_sync();

@@ -7,17 +7,16 @@
 // 500 x 2048 x 7168 35.8 (on CTA pairs) -> 25.5 us.
 #pragma once
 
-#include "gemm_tc.cuh"
+#include "cluster_sum.cuh"
 
 namespace slime {
 namespace gemm {
 
 constexpr int kKsStages     = 4;
-constexpr int kKsBN         = 256;
+constexpr int kKsBN         = kSumCols;
 constexpr int kKsStageBytes = (kBM + kKsBN) * kBK * 2;
-constexpr int kKsSumPitch   = kKsBN + 4;  // floats per row of the sums: 16-byte accesses of eight rows hit all banks
 constexpr int kKsSmem       = kKsStages * kKsStageBytes + (2 * kKsStages + 1) * 8 + 16 + 1024;
-static_assert(kKsStages * kKsStageBytes >= kKsSumPitch * kBM * 4, "the ring holds the sums of the tile afterwards");
+static_assert(kKsStages * kKsStageBytes >= kSumPitch * kBM * 4, "the ring holds the sums of the tile afterwards");
 
 static __global__ void __launch_bounds__(kThreads, 1)
 gemm_bf16_ksplit_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const __grid_constant__ Args args, int split)
@@ -64,7 +63,7 @@ gemm_bf16_ksplit_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_co
     tc_fence_after_sync();
     const uint32_t tmem_base = *tmem_slot;
 
-    float* sums = reinterpret_cast<float*>(smem);  // [128 rows][kKsSumPitch], once the ring has been consumed
+    float* sums = reinterpret_cast<float*>(smem);  // [128 rows][kSumPitch], once the ring has been consumed
     if (warp == 0) {
         // ------------------------------ TMA producer ------------------------------
         for (int i = 0; i < kblocks; ++i) {
@@ -121,34 +120,14 @@ gemm_bf16_ksplit_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_co
                 uint32_t v[32];
                 tmem_ld_32x32b_x32(taddr + c, v);
                 tmem_ld_wait();
-                uint4* dst = reinterpret_cast<uint4*>(sums + trow * kKsSumPitch + c);
+                uint4* dst = reinterpret_cast<uint4*>(sums + trow * kSumPitch + c);
 #pragma unroll
                 for (int i = 0; i < 8; ++i) dst[i] = make_uint4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
             }
         }
     }
 
-    __syncwarp();
-    cluster_sync_all();  // the sums of all CTAs of the cluster are in place
-    {
-        // this CTA's slice of the columns, four at a time: N is a multiple of 32, so four columns exist together or not at all
-        const int quads = kKsBN / split / 4;
-        const int rows  = min(kBM, args.M_total - row0);
-        for (int i = threadIdx.x; i < rows * quads; i += kThreads) {
-            const int r = i / quads;
-            const int c = (crank * quads + i % quads) * 4;
-            if (col0 + c >= args.N) continue;
-            float4 v[8];
-#pragma unroll
-            for (int j = 0; j < 8; ++j)
-                if (j < split) v[j] = ld_cluster_f32x4(mapa_u32(sums + r * kKsSumPitch + c, static_cast<uint32_t>(j)));
-            float4 a = v[0];
-#pragma unroll
-            for (int j = 1; j < 8; ++j)
-                if (j < split) a = make_float4(a.x + v[j].x, a.y + v[j].y, a.z + v[j].z, a.w + v[j].w);
-            *reinterpret_cast<uint2*>(args.C + static_cast<long long>(row0 + r) * args.ldc + col0 + c) = make_uint2(pack_bf16(a.x, a.y), pack_bf16(a.z, a.w));
-        }
-    }
+    cluster_add_store(sums, fail_slot, crank, split, row0, col0, args.M_total, args.N, args.C, args.ldc);
 
     // teardown: no CTA may leave while another one still reads its sums
     tc_fence_before_sync();

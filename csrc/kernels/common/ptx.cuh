@@ -507,6 +507,12 @@ __device__ __forceinline__ uint32_t mapa_u32(const void* ptr, uint32_t rank)
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(out) : "r"(smem_u32(ptr)), "r"(rank));
     return out;
 }
+__device__ __forceinline__ uint32_t ld_cluster_u32(uint32_t cluster_addr)
+{
+    uint32_t v;
+    asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(cluster_addr) : "memory");
+    return v;
+}
 // 16 bytes of another CTA's shared memory (a shared::cluster address from mapa_u32)
 __device__ __forceinline__ float4 ld_cluster_f32x4(uint32_t cluster_addr)
 {

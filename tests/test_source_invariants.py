@@ -86,6 +86,19 @@ def test_waits_of_whole_warps_end_alike_in_all_lanes():
     assert not bad, bad
 
 
+def test_split_products_store_nothing_after_a_wait_that_ran_out():
+    """The kernels that split a product along K over a cluster store through one function, which asks every CTA of the cluster
+    whether it gave up before it adds or stores anything."""
+    common = ROOT / "csrc" / "kernels" / "common"
+    text = {p.name: "\n".join(line for _, line in _code_lines(p)) for p in common.glob("*.cuh")}
+    body = text["cluster_sum.cuh"].split("void cluster_add_store", 1)[1]
+    order = [body.index(s) for s in ("cluster_sync_all()", "ld_cluster_u32", "__any_sync", "return;", "ld_cluster_f32x4", "<uint2*>(C")]
+    assert order == sorted(order)
+    for name in ("gemm_ks.cuh", "gemm_fp8_pair.cuh"):
+        kernel = text[name].split("ksplit_kernel", 1)[1]
+        assert "cluster_add_store(sums, fail_slot" in kernel and "ld_cluster_f32x4" not in kernel, name
+
+
 def test_c_api_header_and_library_agree():
     """Every function declared in the public C headers is exported by the built kernel library."""
     from dlslime_b200 import _lib
