@@ -106,11 +106,11 @@ __device__ __forceinline__ int push_order_expert(const EpConfig& c, int o)
 // ---------------------------------------------------------------------------
 // route: one warp per token
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) ep_route_kernel(EpConfig cfg, const float* __restrict__ logits, int T,
-                                                      int* __restrict__ topk_idx, float* __restrict__ topk_w,
-                                                      int* __restrict__ slot, unsigned int* __restrict__ send_count,
-                                                      unsigned int* __restrict__ block_counter, unsigned long long epoch,
-                                                      int renormalize, int* __restrict__ push_off)
+__global__ void __launch_bounds__(256) ep_route_kernel(EpConfig cfg, const float* logits, int T,
+                                                      int* topk_idx, float* topk_w,
+                                                      int* slot, unsigned int* send_count,
+                                                      unsigned int* block_counter, unsigned long long epoch,
+                                                      int renormalize, int* push_off)
 {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int t    = blockIdx.x * 8 + warp;
@@ -250,11 +250,11 @@ __global__ void __launch_bounds__(256) ep_perm_kernel(EpConfig cfg, int T, const
 // dispatch and 146 us for the receive.
 // ---------------------------------------------------------------------------
 template<bool kExpand>
-__global__ void __launch_bounds__(256) ep_dispatch_kernel(EpConfig cfg, const __nv_bfloat16* __restrict__ x, long long ldx,
-                                                         int T, const int* __restrict__ topk_idx,
-                                                         const int* __restrict__ slot, int* __restrict__ group_offsets,
-                                                         unsigned int* __restrict__ block_counter,
-                                                         __nv_bfloat16* __restrict__ y, long long ldy,
+__global__ void __launch_bounds__(256) ep_dispatch_kernel(EpConfig cfg, const __nv_bfloat16* x, long long ldx,
+                                                         int T, const int* topk_idx,
+                                                         const int* slot, int* group_offsets,
+                                                         unsigned int* block_counter,
+                                                         __nv_bfloat16* y, long long ldy,
                                                          unsigned long long epoch, KernelStatus* st)
 {
     __shared__ unsigned int s_total[kMaxExperts];
@@ -784,9 +784,9 @@ __global__ void ep_signal_kernel(EpConfig cfg, unsigned long long off, unsigned 
     }
 }
 
-__global__ void __launch_bounds__(256) ep_combine_reduce_kernel(EpConfig cfg, int T, const int* __restrict__ topk_idx,
-                                                               const float* __restrict__ topk_w,
-                                                               __nv_bfloat16* __restrict__ out, long long ldo,
+__global__ void __launch_bounds__(256) ep_combine_reduce_kernel(EpConfig cfg, int T, const int* topk_idx,
+                                                               const float* topk_w,
+                                                               __nv_bfloat16* out, long long ldo,
                                                                unsigned long long epoch, int do_signal, KernelStatus* st)
 {
     griddep_wait();
@@ -873,6 +873,8 @@ int check_cfg(const EpConfig& c)
 // Launches one kernel of a step. With one rank nothing in the step waits for a peer, so the kernels are chained as
 // programmatic dependents: each one's blocks are scheduled while the kernel in front of it drains, and wait for its
 // completion first thing. With more ranks a block that only waits could hold a slot that a peer's progress needs.
+// A chained kernel is running while the one in front of it still writes what it is going to read, so its pointers carry no
+// __restrict__, which would promise that nobody does (and allow loads that bypass the coherent path).
 // Three tokens on 32 experts, launched eagerly: 344 -> 336 us a step; no difference where the GEMMs take milliseconds.
 template<typename... KArgs, typename... Args>
 cudaError_t launch_chained(const EpConfig& cfg, void (*kernel)(KArgs...), int grid, cudaStream_t stream, Args&&... args)

@@ -99,6 +99,21 @@ def test_split_products_store_nothing_after_a_wait_that_ran_out():
         assert "cluster_add_store(sums, fail_slot" in kernel and "ld_cluster_f32x4" not in kernel, name
 
 
+def test_chained_kernels_promise_nothing_about_their_inputs():
+    """A kernel that waits for its predecessor inside (griddep_wait) runs while that one still writes: none of its pointers may be
+    declared __restrict__, which says that the data does not change during the kernel's life."""
+    seen, bad = 0, []
+    for p in KERNELS:
+        text = "\n".join(line for _, line in _code_lines(p))
+        for kernel in text.split("__global__")[1:]:
+            signature, body = kernel.split("\n{", 1)
+            if "griddep_wait()" in body:
+                seen += 1
+                if "__restrict__" in signature:
+                    bad.append((p.name, signature[:120]))
+    assert seen >= 6 and not bad, (seen, bad)
+
+
 def test_c_api_header_and_library_agree():
     """Every function declared in the public C headers is exported by the built kernel library."""
     from dlslime_b200 import _lib
