@@ -339,6 +339,14 @@ int check_common(int M, int N, int K, long long lda, long long ldb)
     return 0;
 }
 
+// The epilogues store `bytes` (16; 8 where a form says so) at a time: a row of C that starts elsewhere would fault the GPU.
+int check_out(const void* C, long long ldc, int bytes = 16)
+{
+    if ((reinterpret_cast<unsigned long long>(C) % bytes) != 0 || (ldc * 2) % bytes != 0)
+        return fail("gemm: rows of the output must be %d-byte aligned (C %p, ldc %lld)", bytes, C, ldc);
+    return 0;
+}
+
 }  // namespace
 
 extern "C" {
@@ -348,6 +356,7 @@ int slime_gemm_bf16(const void* A, const void* B, void* C, int M, int N, int K, 
 {
     if (check_common(M, N, K, lda, ldb)) return -1;
     if (ldc % 8 != 0) return fail("gemm: ldc must be a multiple of 8 elements");
+    if (check_out(C, ldc, 8)) return -1;
     Args a{};
     a.M_total    = M;
     a.N          = N;
@@ -358,7 +367,8 @@ int slime_gemm_bf16(const void* A, const void* B, void* C, int M, int N, int K, 
     a.ldc        = ldc;
     a.status     = static_cast<KernelStatus*>(status);
     const int split = pick_ksplit(M, N, K);
-    if (split > 1 && (reinterpret_cast<unsigned long long>(C) & 7) == 0) return launch_ksplit(A, B, a, lda, ldb, split, static_cast<cudaStream_t>(stream));
+    if (split > 1) return launch_ksplit(A, B, a, lda, ldb, split, static_cast<cudaStream_t>(stream));
+    if (check_out(C, ldc)) return -1;
     return launch<kEpiStore>(A, B, a, lda, ldb, static_cast<cudaStream_t>(stream));
 }
 
@@ -368,6 +378,7 @@ int slime_gemm_bf16_pair(const void* A, const void* B, void* C, int M, int N, in
 {
     if (check_common(M, N, K, lda, ldb)) return -1;
     if (ldc % 8 != 0) return fail("gemm: ldc must be a multiple of 8 elements");
+    if (check_out(C, ldc)) return -1;
     Args a{};
     a.M_total    = M;
     a.N          = N;
@@ -386,6 +397,7 @@ int slime_gemm_bf16_wide(const void* A, const void* B, void* C, int M, int N, in
 {
     if (check_common(M, N, K, lda, ldb)) return -1;
     if (ldc % 8 != 0) return fail("gemm: ldc must be a multiple of 8 elements");
+    if (check_out(C, ldc)) return -1;
     Args a{};
     a.M_total    = M;
     a.N          = N;
@@ -404,6 +416,7 @@ int slime_gemm_bf16_gated(const void* A, const void* B, void* C, int M, int N, i
 {
     if (check_common(M, N, K, lda, ldb)) return -1;
     if (a_ready && (a_ready_rows <= 0)) return fail("gemm: a_ready_rows must be positive");
+    if (check_out(C, ldc)) return -1;
     Args a{};
     a.M_total        = M;
     a.N              = N;
@@ -460,6 +473,7 @@ int slime_ag_gemm(int mode, const void* x_local, const void* a_full, const void*
         return 0;
     }
     if (check_common(a.M_total, N, K, K, ldb)) return -1;
+    if (check_out(C, ldc)) return -1;
     a.a_ready        = reinterpret_cast<const unsigned long long*>(flags8[rank]);
     a.a_ready_rows   = kBM;
     a.a_ready_target = step * (kBM / kAgSliceRows);
@@ -540,8 +554,6 @@ int slime_grouped_gemm_bf16_wt(const void* A, const void* B, void* C, const int*
 {
     if (tile_tokens != 64 && tile_tokens != 128 && tile_tokens != 192) return fail("grouped gemm: tiles of %d tokens are not offered", tile_tokens);
     if (chained < 0 || chained > 2) return fail("grouped gemm: chained = %d not in [0, 2]", chained);
-    if (epilogue != kEpiScatterRows && (ldc % 8 != 0 || (reinterpret_cast<unsigned long long>(C) & 15) != 0))
-        return fail("grouped gemm: rows of the output must be 16-byte aligned");
     g_wt_tokens  = tile_tokens;
     g_chained    = chained;
     const int rc = grouped_gemm_impl(A, B, C, group_offsets, num_groups, M_cap, N, K, lda, ldb, ldc, epilogue, row_info, scatter_bases8,
@@ -641,6 +653,7 @@ static int grouped_gemm_impl(const void* A, const void* B, void* C, const int* g
 {
     if (check_common(M_cap, N, K, lda, ldb)) return -1;
     if (num_groups <= 0 || group_offsets == nullptr) return fail("grouped gemm: need group offsets");
+    if (epilogue != kEpiScatterRows && check_out(C, ldc, g_on_pairs == 3 ? 8 : 16)) return -1;  // the swapped pairs store 8 bytes at a time
     Args a{};
     a.group_ready        = group_ready;
     a.group_ready_target = group_ready_target;
@@ -678,7 +691,10 @@ static int grouped_gemm_impl(const void* A, const void* B, void* C, const int* g
             a.rowsB     = N;
             a.row_info  = static_cast<const unsigned long long*>(row_info);
             a.row_scale = row_scale;
-            for (int i = 0; i < 8; ++i) a.scatter_base[i] = scatter_bases8[i];
+            for (int i = 0; i < 8; ++i) {
+                if (scatter_bases8[i] % (g_on_pairs == 3 ? 8 : 16) != 0) return fail("grouped gemm: scatter rows must be 16-byte aligned");
+                a.scatter_base[i] = scatter_bases8[i];
+            }
             a.scatter_row_bytes = scatter_row_bytes;
             a.scatter_slots     = scatter_slots;
             if (g_wt_tokens) return launch_wt<kEpiScatterRows>(g_wt_tokens, A, B, a, lda, ldb, s);
@@ -700,6 +716,7 @@ int slime_grouped_gemm_fp8a(const void* Aq, const float* a_scale, const void* B,
     if (check_common(M_cap, N, K, 8, ldb)) return -1;
     if (K % 128 != 0 || lda_bytes % 16 != 0) return fail("fp8-A grouped gemm: K must be a multiple of 128 and lda of 16 bytes");
     if (num_groups <= 0 || group_offsets == nullptr || a_scale == nullptr) return fail("fp8-A grouped gemm: need group offsets and scales");
+    if (check_out(C, ldc)) return -1;
     Args a{};
     a.M_total       = M_cap;
     a.N             = N;

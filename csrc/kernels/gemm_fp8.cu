@@ -100,6 +100,7 @@ int launch_plain_f8(const void* Aq, const void* Bq, const F8Args& g, long long l
         SLIME_CUDA_OK(cudaLaunchKernelEx(&cfg, gemm_fp8_ksplit_kernel, tmA, tmB, f));
         return 0;
     }
+    if (reinterpret_cast<unsigned long long>(f.C) % 16 != 0) return fail("fp8 gemm: the output must be 16-byte aligned (%p)", static_cast<void*>(f.C));
     if (f.M <= kBM) return launch_f8<false>(Aq, Bq, nullptr, g, lda, ldb, stream);
     const int  pairs      = sms / 2;
     const long pair_tiles = static_cast<long>((f.M + 2 * kBM - 1) / (2 * kBM)) * ntiles;
@@ -119,12 +120,13 @@ int launch_plain_f8(const void* Aq, const void* Bq, const F8Args& g, long long l
     return 0;
 }
 
-int check_f8(int M, int N, int K, long long lda, long long ldb, long long ldc)
+int check_f8(const void* C, int M, int N, int K, long long lda, long long ldb, long long ldc, int out_align = 16)
 {
     if (M <= 0 || N <= 0 || K <= 0) return fail("fp8 gemm: M, N, K must be positive (got %d, %d, %d)", M, N, K);
     if (K % kF8BK != 0) return fail("fp8 gemm: K (%d) must be a multiple of %d (one scale block)", K, kF8BK);
     if (lda % 16 != 0 || ldb % 16 != 0) return fail("fp8 gemm: lda and ldb must be multiples of 16 bytes");
     if (N % 32 != 0 || ldc % 8 != 0) return fail("fp8 gemm: N must be a multiple of 32 and ldc of 8");
+    if (reinterpret_cast<unsigned long long>(C) % out_align != 0) return fail("fp8 gemm: the output must be %d-byte aligned (%p)", out_align, C);
     return 0;
 }
 
@@ -136,7 +138,7 @@ extern "C" {
 int slime_gemm_fp8_blockscaled(const void* Aq, const float* sa, const void* Bq, const float* sb, void* C, int M, int N, int K,
                                long long lda, long long ldb, long long ldc, void* status, void* stream)
 {
-    if (check_f8(M, N, K, lda, ldb, ldc)) return -1;
+    if (check_f8(C, M, N, K, lda, ldb, ldc, 8)) return -1;  // 16 where the form stores 16 bytes at a time, see launch_plain_f8
     F8Args f{};
     f.M = M;
     f.N = N;
@@ -191,7 +193,7 @@ int slime_ag_gemm_fp8(int mode, const void* xq_local, const float* sx_local, con
         SLIME_CUDA_OK(cudaGetLastError());
         return 0;
     }
-    if (check_f8(f.M, N, K, K, ldb, ldc)) return -1;
+    if (check_f8(C, f.M, N, K, K, ldb, ldc)) return -1;
     f.ag.a_ready        = reinterpret_cast<const unsigned long long*>(flags8[rank]);
     f.ag.a_ready_rows   = kBM;
     f.ag.a_ready_target = step * (kBM / kAgSliceRows);
