@@ -52,11 +52,8 @@ int launch_bn(const void* A, const void* B, const void* A_local, int rows_local,
         tmAL = tmA;
     }
     auto kern = gemm_bf16_tc_kernel<BN, STAGES, EPI, AG, false, AROWS>;
-    static bool configured = false;
-    if (!configured) {
-        SLIME_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, S::kTotal));
-        configured = true;
-    }
+    static bool configured[64] = {};
+    SLIME_CUDA_OK(allow_dynamic_smem(kern, S::kTotal, configured));
     const long tiles = static_cast<long>((args.M_total + AROWS - 1) / AROWS) * ((args.N + BN - 1) / BN);
     int        grid  = sm_count();
     // a fused all-gather kernel keeps the full grid (its extra warps push whatever the tile count is);
@@ -165,11 +162,8 @@ int launch_a8(const void* Aq, const void* B, const Args& args, long long lda_byt
     if (make_tmap_2d(&tmA, Aq, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, args.M_total, args.K, lda_bytes, kBM, kBK)) return -1;
     if (make_tmap_2d(&tmB, B, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, rowsB_total, args.K, ldb, kBN / 2, kBK)) return -1;
     auto kern = gemm_bf16_tc_kernel<kBN, kStagesA8, EPI, false, true>;
-    static bool configured = false;
-    if (!configured) {
-        SLIME_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, S::kTotal));
-        configured = true;
-    }
+    static bool configured[64] = {};
+    SLIME_CUDA_OK(allow_dynamic_smem(kern, S::kTotal, configured));
     kern<<<sm_count(), kThreads + kCvtThreads, S::kTotal, stream>>>(tmA, tmB, tmA, args);
     SLIME_CUDA_OK(cudaGetLastError());
     return 0;
@@ -207,11 +201,8 @@ int launch_pair_bn(const void* A, const void* B, const void* A_local, const Args
         tmAL = tmA;
     }
     auto kern = gemm_bf16_pair_kernel<BN, STAGES, AG>;
-    static bool configured = false;
-    if (!configured) {
-        SLIME_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, S::kTotal));
-        configured = true;
-    }
+    static bool configured[64] = {};
+    SLIME_CUDA_OK(allow_dynamic_smem(kern, S::kTotal, configured));
     const long tiles    = static_cast<long>((args.M_total + kPairBM - 1) / kPairBM) * ((args.N + BN - 1) / BN);
     int        clusters = sm_count() / 2;
     if (!AG && tiles < clusters) clusters = static_cast<int>(tiles);
@@ -241,11 +232,8 @@ int launch_pair_grouped(const void* A, const void* B, const Args& args, long lon
     if (make_tmap_2d(&tmA, A, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, args.M_total, args.K, lda, kBM, kBK)) return -1;
     if (make_tmap_2d(&tmB, B, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, rowsB_total, args.K, ldb, kBN / 2, kBK)) return -1;
     auto kern = gemm_bf16_pair_grouped_kernel<kBN, kPairStages, EPI>;
-    static bool configured = false;
-    if (!configured) {
-        SLIME_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, S::kTotal));
-        configured = true;
-    }
+    static bool configured[64] = {};
+    SLIME_CUDA_OK(allow_dynamic_smem(kern, S::kTotal, configured));
     kern<<<2 * (sm_count() / 2), kThreads, S::kTotal, stream>>>(tmA, tmB, args);
     SLIME_CUDA_OK(cudaGetLastError());
     return 0;
@@ -262,11 +250,8 @@ int launch_pair_swapped(const void* A, const void* B, const Args& args, long lon
     if (make_tmap_2d(&tmX, A, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, args.M_total, args.K, lda, kBM, kBK)) return -1;
     if (make_tmap_2d(&tmW, B, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, rowsB_total, args.K, ldb, EPI == kEpiSwiGLU ? kBM / 2 : kBM, kBK)) return -1;
     auto kern = gemm_bf16_pair_swapped_kernel<kSwapStages, EPI>;
-    static bool configured = false;
-    if (!configured) {
-        SLIME_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, S::kTotal));
-        configured = true;
-    }
+    static bool configured[64] = {};
+    SLIME_CUDA_OK(allow_dynamic_smem(kern, S::kTotal, configured));
     kern<<<2 * (sm_count() / 2), kThreads, S::kTotal, stream>>>(tmW, tmX, args);
     SLIME_CUDA_OK(cudaGetLastError());
     return 0;
@@ -283,11 +268,8 @@ int launch_pair_wide(const void* A, const void* B, const Args& args, long long l
     if (make_tmap_2d(&tmA, A, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, args.M_total, args.K, lda, kBM, kBK)) return -1;
     if (make_tmap_2d(&tmB, B, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, rowsB_total, args.K, ldb, kBN / 2, kBK)) return -1;
     auto kern = gemm_bf16_pair_wide_kernel<kBN, kWideStages, EPI>;
-    static bool configured = false;
-    if (!configured) {
-        SLIME_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, S::kTotal));
-        configured = true;
-    }
+    static bool configured[64] = {};
+    SLIME_CUDA_OK(allow_dynamic_smem(kern, S::kTotal, configured));
     int clusters = sm_count() / 2;
     if (args.group_offsets == nullptr) {
         constexpr int kTileOut = EPI == kEpiSwiGLU ? kBN : 2 * kBN;

@@ -37,11 +37,8 @@ int launch_f8(const void* Aq, const void* Bq, const void* A_local, const F8Args&
         tmAL = tmA;
     }
     auto kern = gemm_fp8_blockscaled_kernel<AG>;
-    static bool configured = false;
-    if (!configured) {
-        SLIME_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, S::kTotal));
-        configured = true;
-    }
+    static bool configured[64] = {};
+    SLIME_CUDA_OK(allow_dynamic_smem(kern, S::kTotal, configured));
     const long tiles = static_cast<long>((f.M + kBM - 1) / kBM) * ((f.N + kF8BN - 1) / kF8BN);
     int        grid  = sm_count();
     if (!AG && tiles < grid) grid = static_cast<int>(tiles);

@@ -114,6 +114,13 @@ def test_chained_kernels_promise_nothing_about_their_inputs():
     assert seen >= 6 and not bad, (seen, bad)
 
 
+def test_function_attributes_are_remembered_per_device():
+    """A function attribute belongs to one device's copy of the kernel, and a process may drive several devices: what remembers
+    that it has been set is an array over devices, never one word for the process."""
+    bad = [(p.name, i) for p in KERNELS for i, line in _code_lines(p) if re.search(r"static\s+bool\s+\w+\s*(=|;|\{)", line)]
+    assert not bad, bad
+
+
 def test_c_api_header_and_library_agree():
     """Every function declared in the public C headers is exported by the built kernel library."""
     from dlslime_b200 import _lib
