@@ -19,7 +19,9 @@ oracle.
 
 from __future__ import annotations
 
+import os
 from dataclasses import dataclass
+from typing import NamedTuple
 
 import torch
 
@@ -57,6 +59,47 @@ def init_expert_weights(cfg: MoEConfig, experts: range, device, seed: int = 0):
     return w13, w2
 
 
+class ExpertGemmForm(NamedTuple):
+    """Which of the grouped GEMM's forms the expert FFN takes (the arguments of :func:`gemm.grouped_gemm_bf16`)."""
+
+    pair: bool | str  # False: single CTAs; True: CTA pairs, 256 x 256 tiles; "wide": 256 x 512; "swap": weights on the M side
+    tile_n: int       # single CTAs, tokens on the M side: tile width (0 = 256)
+    tile_m: int       # the same: row tiles of 64 (0 = 128)
+    tile_tokens: int  # single CTAs, weights on the M side: most rows of a group per tile (0 = tokens on the M side)
+
+
+def expert_gemm_form(rows: float, env=None) -> ExpertGemmForm:
+    """The form for experts that expect ``rows`` rows each in a step.
+
+    Measured at hidden 7168, intermediate 2048 on one rank, whole steps run back to back (other widths and more ranks take the
+    same lines). Below ``gemm.WT_MAX_ROWS`` rows the weights go on the M side of single CTAs (:func:`gemm.pick_tile_tokens`), from there to
+    ``gemm.SWAP_MAX_ROWS`` on the M side of CTA pairs. Then come 128-row tiles, and from 1024 rows pairs, whose larger tiles waste
+    little there: 2815 us a step against 2860 on single CTAs with 32 x 1024 rows, but 3775 against 3300 with 64 x 512 and 3085
+    against 2744 with 64 x 384.
+
+    The environment overrides the rule: SLIME_EP_PAIR_GEMM=0|1|wide|swap the kind; SLIME_EP_TILE_N, SLIME_EP_TILE_M=0|64 and
+    SLIME_EP_TILE_TOKENS=0|64|128|192 the tiles of the single-CTA forms, so none of them goes with "swap" unless that is forced.
+    Narrower tiles (SLIME_EP_TILE_N) do not pay for decode-size steps on many ranks (32 experts x 32 rows: 512 tiles = 3.46 waves of
+    the grid): those GEMMs stream weights from HBM, the CTAs do not wait for one another between waves, and a short last wave
+    still fills the memory system (5.66 TB/s of weights with 256-wide tiles, 5.53 with the widths that fill the waves). Row
+    tiles of 64 are for groups of a few dozen rows with the tokens on the M side, so they matter only where SLIME_EP_TILE_TOKENS=0.
+    """
+    env = os.environ if env is None else env
+    kind, tile_n = env.get("SLIME_EP_PAIR_GEMM"), int(env.get("SLIME_EP_TILE_N", "0"))
+    tile_m, tile_tokens = env.get("SLIME_EP_TILE_M"), env.get("SLIME_EP_TILE_TOKENS")
+    tiles_given = bool(tile_n) or tile_m is not None or tile_tokens is not None
+    if kind is not None:
+        pair = {"0": False, "1": True}.get(kind, kind)
+    elif gemm.WT_MAX_ROWS <= rows < gemm.SWAP_MAX_ROWS and not tiles_given:
+        pair = "swap"
+    else:
+        pair = rows >= 1024
+    few_rows = 64 if rows + 3 * rows ** 0.5 <= 64 else 0
+    free = not tile_n and tile_m is None
+    return ExpertGemmForm(pair, tile_n, few_rows if tile_m is None else int(tile_m),
+                          int(tile_tokens) if tile_tokens is not None else gemm.pick_tile_tokens(rows) if free else 0)
+
+
 class ExpertParallelMoE:
     """One rank's shard of the MoE layer."""
 
@@ -82,35 +125,14 @@ class ExpertParallelMoE:
         # streamed: dispatch, receive and the gate/up GEMM run at the same time (see forward_streamed)
         self.streamed = streamed and not fuse_dequant
         # grid of the streamed form's push + receive kernel (0 = three blocks per SM; a multiple of 3)
-        import os
-
         self.comm_blocks = int(os.environ.get("SLIME_EP_COMM_BLOCKS", "0"))
         # words of the gated GEMM's dynamic tile scheduler (SLIME_EP_STATIC_TILES=1: every gridDim-th tile instead)
         self._tile_counter = None if os.environ.get("SLIME_EP_STATIC_TILES") == "1" else torch.zeros(2, dtype=torch.int32, device=dev)
-        # pair_gemm: the expert GEMMs on CTA pairs (True: 256 x 256 tiles, "wide": 256 x 512). They win where a local
-        # expert sees a thousand rows per step (many ranks) and their larger tiles waste little: steps run back to back at the
-        # power limit take 2815 us against 2860 on single CTAs with 32 x 1024 rows, but 3775 against 3300 with 64 x 512 and 3085 against
-        # 2744 with 64 x 384. "swap" (weights on the M side of a pair) wins between 176 and 320 rows, see gemm.pick_tile_tokens;
-        # SLIME_EP_PAIR_GEMM=0|1|wide|swap overrides the rule, autotune() measures.
-        rows_per_expert = max_tokens * cfg.topk * self.world // max(1, cfg.num_experts)
-        forced = os.environ.get("SLIME_EP_PAIR_GEMM")
-        swap = gemm.WT_MAX_ROWS <= rows_per_expert < gemm.SWAP_MAX_ROWS
-        self.pair_gemm = (rows_per_expert >= 1024 or (swap and "swap")) if forced is None else {"0": False, "1": True}.get(forced, forced)
-        # tile width of the single-CTA expert GEMMs (0 = 256). Narrower tiles were measured for the decode-size step on
-        # many ranks (32 experts x 32 rows: 512 tiles = 3.46 waves of the grid) and do not pay: those GEMMs stream weights
-        # from HBM, the CTAs do not wait for one another between waves, and a short last wave still fills the memory
-        # system (5.66 TB/s of weights with 256-wide tiles, 5.53 with the widths that fill the waves).
-        self.tile_n_gate_up = self.tile_n_down = int(os.environ.get("SLIME_EP_TILE_N", "0"))
-        # with the tokens on the M side (tile_tokens = 0 below): row tiles of 64 where a local expert is expected to see a few dozen rows per step (decode steps): the A part of
-        # a pipeline stage halves, the ring gets a fifth stage and more weight bytes are in flight (SLIME_EP_TILE_M=0|64)
-        expected = max_tokens * cfg.topk * self.world / max(1, cfg.num_experts)
-        forced_m = os.environ.get("SLIME_EP_TILE_M")
-        self.tile_m = (64 if expected + 3 * expected ** 0.5 <= 64 else 0) if forced_m is None else int(forced_m)
-        # weights on the M side, a group's rows on the N side (SLIME_EP_TILE_TOKENS=0|64|128|192); autotune's other kinds and the
-        # tile overrides above take precedence
-        forced_t = os.environ.get("SLIME_EP_TILE_TOKENS")
-        free = not self.tile_n_gate_up and forced_m is None
-        self.tile_tokens = int(forced_t) if forced_t is not None else gemm.pick_tile_tokens(expected) if free else 0
+        # pair_gemm, tile_n_*, tile_m, tile_tokens: see expert_gemm_form; autotune() measures and sets pair_gemm
+        form = expert_gemm_form(max_tokens * cfg.topk * self.world / max(1, cfg.num_experts))
+        self._default_pair_gemm = self.pair_gemm = form.pair
+        self.tile_n_gate_up = self.tile_n_down = form.tile_n
+        self.tile_m, self.tile_tokens = form.tile_m, form.tile_tokens
         cap = self.buf.recv_cap
         self.xd = torch.empty((cap, cfg.hidden), dtype=torch.bfloat16, device=dev)
         self.h = torch.empty((cap, cfg.intermediate), dtype=torch.bfloat16, device=dev)
@@ -211,58 +233,57 @@ class ExpertParallelMoE:
         return out
 
     def autotune(self, x: torch.Tensor, logits: torch.Tensor, out: torch.Tensor | None = None, steps: int = 4) -> dict:
-        """Pick the faster expert GEMM (single CTAs or CTA pairs) and then the faster of the two forms of the first half
-        (phases one after the other, or streamed) for this shape and world size by running them, and keep both. A form
-        replaces the default (single CTAs, phases one after the other) only if it wins by more than 1 %, so that
-        run-to-run noise does not pick. Every rank must call this with its own inputs of the step shape; the device times
+        """Pick the fastest expert GEMM (the layer's own choice of :func:`expert_gemm_form`, single CTAs, CTA pairs) and then the
+        faster of the two forms of the first half (phases one after the other, or streamed) for this shape and world size by
+        running them, and keep both. A form replaces the default (the layer's own choice, phases one after the other) only if
+        it wins by more than 1 %, so that run-to-run noise does not pick. Every rank must call this with its own inputs of the step shape; the device times
         are combined as the maximum over ranks, so all ranks decide alike. Which form wins
         depends on the regime: streaming hides the NVLink-bound push under compute-bound expert GEMMs (many ranks, many
         rows per expert) and loses where the GEMMs stream weights from HBM and the extra traffic gets in their way.
         """
-        import torch.distributed as dist
-
         if self.fuse_dequant:
             return {"streamed": False, "reason": "the fused-dequant GEMM has no streamed form"}
-        times = {}
-        # wide pairs and swapped operands have lost on every shape measured so far (1, 2 and 8 GPUs): they are timed only
-        # on request
-        import os
-
-        kinds = {"single": False, "pair": True}
+        names = {False: "single", True: "pair", "wide": "wide", "swap": "swap"}
+        default = names.get(self._default_pair_gemm, "pair")
+        # beside the layer's own choice: the wide and swapped pairs only on request
+        kinds = {default: self._default_pair_gemm, "single": False, "pair": True}
         if os.environ.get("SLIME_EP_AUTOTUNE_ALL") == "1":
             kinds.update({"wide": "wide", "swap": "swap"})
-        for form in (*kinds, True):
-            if form is True:
-                best = min(kinds, key=lambda k: times[k])
-                if times[best] > 0.99 * times["single"]:
-                    best = "single"
-                self.pair_gemm = kinds[best]
-                times[False] = times[best]
-            self.streamed = form is True
-            if form is not True:
-                self.pair_gemm = kinds[form]
-            for _ in range(2):
-                self.forward(x, logits, out)
-            if dist.is_initialized():
-                dist.barrier()
-            torch.cuda.synchronize()
-            e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
-            e0.record()
-            for _ in range(steps):
-                self.forward(x, logits, out)
-            e1.record()
-            torch.cuda.synchronize()
-            t = torch.tensor([e0.elapsed_time(e1) / steps], device=x.device, dtype=torch.float64)
-            if dist.is_initialized() and dist.get_world_size() > 1:
-                dist.all_reduce(t, op=dist.ReduceOp.MAX)
-            times[form] = float(t.item())
-            self.buf.status.check()
-        self.streamed = times[True] < 0.99 * times[False]
-        return {"streamed": self.streamed, "pair_gemm": self.pair_gemm, "serial_ms": round(times[False], 4),
-                "serial_single_cta_ms": round(times["single"], 4), "serial_cta_pair_ms": round(times["pair"], 4),
-                **({"serial_cta_pair_wide_ms": round(times["wide"], 4), "serial_cta_pair_swapped_ms": round(times["swap"], 4)}
-                   if "wide" in times else {}),
-                "streamed_ms": round(times[True], 4)}
+        times = {}
+        self.streamed = False
+        for name, self.pair_gemm in kinds.items():
+            times[name] = self._time_step(x, logits, out, steps)
+        best = min(times, key=times.get)
+        if times[best] > 0.99 * times[default]:
+            best = default
+        self.pair_gemm, serial = kinds[best], times[best]
+        self.streamed = True
+        streamed = self._time_step(x, logits, out, steps)
+        self.streamed = streamed < 0.99 * serial
+        keys = {"single": "serial_single_cta_ms", "pair": "serial_cta_pair_ms", "wide": "serial_cta_pair_wide_ms", "swap": "serial_cta_pair_swapped_ms"}
+        return {"streamed": self.streamed, "pair_gemm": self.pair_gemm, "serial_ms": round(serial, 4),
+                **{keys[name]: round(t, 4) for name, t in times.items()}, "streamed_ms": round(streamed, 4)}
+
+    def _time_step(self, x, logits, out, steps: int) -> float:
+        """Device milliseconds of one step as the layer is set now, maximum over ranks."""
+        import torch.distributed as dist
+
+        for _ in range(2):
+            self.forward(x, logits, out)
+        if dist.is_initialized():
+            dist.barrier()
+        torch.cuda.synchronize()
+        e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        e0.record()
+        for _ in range(steps):
+            self.forward(x, logits, out)
+        e1.record()
+        torch.cuda.synchronize()
+        t = torch.tensor([e0.elapsed_time(e1) / steps], device=x.device, dtype=torch.float64)
+        if dist.is_initialized() and dist.get_world_size() > 1:
+            dist.all_reduce(t, op=dist.ReduceOp.MAX)
+        self.buf.status.check()
+        return float(t.item())
 
     def forward(self, x: torch.Tensor, logits: torch.Tensor, out: torch.Tensor | None = None) -> torch.Tensor:
         """x [T, hidden] bf16, router logits [T, num_experts] fp32 -> [T, hidden] bf16."""

@@ -1,0 +1,63 @@
+"""Which form of the grouped GEMM the MoE layer takes: the rule by rows per expert, its overrides, and what autotune() keeps."""
+import pytest
+
+from dlslime_b200.models.moe import ExpertGemmForm, ExpertParallelMoE, expert_gemm_form
+
+RULE = {1: ExpertGemmForm(False, 0, 64, 64), 32: ExpertGemmForm(False, 0, 64, 64), 64: ExpertGemmForm(False, 0, 0, 128),
+        128: ExpertGemmForm(False, 0, 0, 192), 175.9: ExpertGemmForm(False, 0, 0, 192), 176: ExpertGemmForm("swap", 0, 0, 0),
+        200: ExpertGemmForm("swap", 0, 0, 0), 300: ExpertGemmForm("swap", 0, 0, 0), 320: ExpertGemmForm(False, 0, 0, 0),
+        500: ExpertGemmForm(False, 0, 0, 0), 1023: ExpertGemmForm(False, 0, 0, 0), 1024: ExpertGemmForm(True, 0, 0, 0)}
+
+
+@pytest.mark.parametrize("rows,form", RULE.items())
+def test_rule_by_rows_per_expert(rows, form):
+    assert expert_gemm_form(rows, {}) == form
+
+
+@pytest.mark.parametrize("rows", [40, 200, 500])
+def test_overrides_are_taken_in_every_range(rows):
+    """A tile override is one of the single-CTA forms, so it also holds where swapped pairs would be the default."""
+    assert expert_gemm_form(rows, {"SLIME_EP_TILE_TOKENS": "128"})[::3] == (False, 128)
+    assert expert_gemm_form(rows, {"SLIME_EP_TILE_N": "192"})[:2] == (False, 192)
+    assert expert_gemm_form(rows, {"SLIME_EP_TILE_N": "192"}).tile_tokens == 0
+    assert expert_gemm_form(rows, {"SLIME_EP_TILE_M": "64"})[:3] == (False, 0, 64)
+    assert expert_gemm_form(rows, {"SLIME_EP_PAIR_GEMM": "0"}).pair is False
+    assert expert_gemm_form(rows, {"SLIME_EP_PAIR_GEMM": "1"}).pair is True
+    assert expert_gemm_form(rows, {"SLIME_EP_PAIR_GEMM": "swap", "SLIME_EP_TILE_M": "0"}).pair == "swap"
+
+
+class _Timed(ExpertParallelMoE):
+    """The layer without a GPU: a step takes what the table says for the form that is set."""
+
+    def __init__(self, rows, times):
+        form = expert_gemm_form(rows, {})
+        self._default_pair_gemm = self.pair_gemm = form.pair
+        self.tile_tokens, self.fuse_dequant, self.streamed = form.tile_tokens, False, False
+        self.times, self.timed = times, []
+
+    def _time_step(self, x, logits, out, steps):
+        self.timed.append("streamed" if self.streamed else self.pair_gemm)
+        return self.times[self.timed[-1]]
+
+
+@pytest.mark.parametrize("rows,times,pair,streamed", [
+    (200, {"swap": 2.64, False: 3.14, True: 3.00, "streamed": 3.2}, "swap", False),   # the layer's own choice is one of the candidates
+    (200, {"swap": 2.64, False: 2.62, True: 3.00, "streamed": 2.65}, "swap", False),  # less than 1 % does not replace it
+    (200, {"swap": 2.64, False: 2.50, True: 3.00, "streamed": 2.4}, False, True),
+    (1024, {False: 2.81, True: 2.82, "streamed": 2.9}, True, False),
+    (128, {False: 4.7, True: 5.4, "streamed": 5.0}, False, False),
+])
+def test_autotune_keeps_the_layers_choice_unless_another_form_wins(rows, times, pair, streamed):
+    layer = _Timed(rows, times)
+    got = layer.autotune(None, None)
+    assert layer.timed[0] == layer._default_pair_gemm and {False, True} <= set(layer.timed)
+    assert layer.pair_gemm is pair or layer.pair_gemm == pair
+    assert layer.streamed is streamed and got["streamed"] is streamed and got["pair_gemm"] == layer.pair_gemm
+    assert got["serial_ms"] == times[pair] and got["streamed_ms"] == times["streamed"]
+
+
+def test_autotune_times_every_form_on_request(monkeypatch):
+    monkeypatch.setenv("SLIME_EP_AUTOTUNE_ALL", "1")
+    layer = _Timed(500, {"swap": 3.0, False: 3.0, True: 3.5, "wide": 2.5, "streamed": 3.0})
+    assert layer.autotune(None, None)["serial_cta_pair_wide_ms"] == 2.5 and layer.pair_gemm == "wide"
+    assert layer.timed == [False, True, "wide", "swap", "streamed"]
