@@ -333,6 +333,13 @@ int check_out(const void* C, long long ldc, int bytes = 16)
 
 extern "C" {
 
+// CTAs that slime_gemm_bf16 would put on each tile of a product of this size (see pick_ksplit); 1: no cluster.
+int slime_gemm_bf16_clusters(int M, int N, int K)
+{
+    if (M <= 0 || N <= 0 || K <= 0) return fail("gemm: M, N, K must be positive (got %d, %d, %d)", M, N, K);
+    return pick_ksplit(M, N, K);
+}
+
 int slime_gemm_bf16(const void* A, const void* B, void* C, int M, int N, int K, long long lda, long long ldb,
                     long long ldc, void* status, void* stream)
 {

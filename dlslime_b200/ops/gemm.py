@@ -57,8 +57,8 @@ def gemm_bf16(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor | None = None,
     if out is None:
         out = torch.empty((m, n), dtype=torch.bfloat16, device=a.device)
     if pair is None:
-        few = -(-m // 128) * -(-n // 256) <= 37 and k >= 2048  # four CTAs a tile still fit, and each has eight K blocks
-        pair = m >= 256 and not few  # two SMs per 256-row tile pay off as soon as there is a full tile
+        # two SMs per 256-row tile pay off as soon as there is a full tile, unless the launcher would share a deep product's K
+        pair = m >= 256 and not (k >= 2048 and _lib.call("slime_gemm_bf16_clusters", m, n, k) > 1)
     if pair:
         return gemm_bf16_pair(a, b, out)
     _lib.call("slime_gemm_bf16", ptr(a), ptr(b), ptr(out), m, n, k, a.stride(0), b.stride(0), out.stride(0),

@@ -1,4 +1,4 @@
-"""Which form of the grouped GEMM the MoE layer takes: the rule by rows per expert, its overrides, and what autotune() keeps."""
+"""Which form of a GEMM is taken: the MoE layer's rule by rows per expert, its overrides, what autotune() keeps, and the plain product."""
 import pytest
 
 from dlslime_b200.models.moe import ExpertGemmForm, ExpertParallelMoE, expert_gemm_form
@@ -61,3 +61,22 @@ def test_autotune_times_every_form_on_request(monkeypatch):
     layer = _Timed(500, {"swap": 3.0, False: 3.0, True: 3.5, "wide": 2.5, "streamed": 3.0})
     assert layer.autotune(None, None)["serial_cta_pair_wide_ms"] == 2.5 and layer.pair_gemm == "wide"
     assert layer.timed == [False, True, "wide", "swap", "streamed"]
+
+
+@pytest.mark.parametrize("clusters,m,k,entry", [(4, 500, 7168, "slime_gemm_bf16"), (1, 500, 7168, "slime_gemm_bf16_pair"), (4, 500, 1024, "slime_gemm_bf16_pair"),
+                                                (4, 255, 1024, "slime_gemm_bf16"), (1, 72, 7168, "slime_gemm_bf16")])
+def test_products_of_few_tiles_follow_the_launchers_rule(monkeypatch, clusters, m, k, entry):
+    """gemm_bf16 asks the launcher whether it would share a tile's K over a cluster; where it would not (clusters that do not fit, a
+    smaller device) a product with a full 256-row tile goes to CTA pairs."""
+    import torch
+
+    from dlslime_b200.ops import gemm
+
+    calls = []
+    monkeypatch.setattr(gemm, "require_cuda", lambda *t: None)
+    monkeypatch.setattr(gemm, "ptr", lambda t: 0)
+    monkeypatch.setattr(gemm, "stream_ptr", lambda *a: 0)
+    monkeypatch.setattr(gemm, "default_status", lambda: type("S", (), {"dev_ptr": 0}))
+    monkeypatch.setattr(gemm._lib, "call", lambda name, *a: clusters if name == "slime_gemm_bf16_clusters" else calls.append(name))
+    gemm.gemm_bf16(torch.empty(m, k, dtype=torch.bfloat16), torch.empty(2048, k, dtype=torch.bfloat16))
+    assert calls == [entry]
