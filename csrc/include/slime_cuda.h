@@ -232,8 +232,16 @@ int slime_ag_wait(const void* cfg_bytes, unsigned long long step, void* status, 
 // ---- paged KV-cache transfer / pack / unpack (kv_transfer.cu) -----------------
 // Moves K and V of one layer for n_tasks pages between a token-major plane pair and a paged plane
 // pair (addresses as integers; the paged side may be peer memory). to_paged: token-major -> paged.
-// threads per CTA of the transfer kernel for the whole process (32 .. 256, a multiple of 32; default 256)
+// threads per CTA of the register form, where a call names none, for the whole process (32 .. 256, a multiple of 32; default 256)
 int slime_kv_tune(int threads);
+// How a call moves its bytes: through registers (CTAs without shared memory, which fit beside a GEMM's), or through the
+// bulk-copy engine (192 KB of shared memory a CTA); auto: bulk copies for pages of 16 KB and more.
+enum { SLIME_KV_AUTO = 0, SLIME_KV_REGISTERS = 1, SLIME_KV_BULK = 2 };
+int slime_kv_transfer_form(unsigned long long tok_k, unsigned long long tok_v, unsigned long long page_k,
+                           unsigned long long page_v, const int* tok_off, const int* blk, const int* ntok, int n_tasks,
+                           int page_tokens, unsigned long long row_bytes, unsigned long long tok_rows,
+                           unsigned long long page_blocks, int to_paged, void* done_flag, unsigned long long done_value,
+                           unsigned int* block_counter, int max_blocks, int form, int threads, void* status, void* stream);
 int slime_kv_transfer(unsigned long long tok_k, unsigned long long tok_v, unsigned long long page_k,
                       unsigned long long page_v, const int* tok_off, const int* blk, const int* ntok, int n_tasks,
                       int page_tokens, unsigned long long row_bytes, unsigned long long tok_rows,

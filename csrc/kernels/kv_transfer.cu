@@ -25,6 +25,8 @@
 #include "common/ptx.cuh"
 #include "slime_cuda.h"
 
+#include <atomic>
+
 using namespace slime;
 
 namespace {
@@ -258,19 +260,24 @@ __global__ void __launch_bounds__(32) kv_bulk_kernel(const __grid_constant__ KvA
     }
 }
 
-int g_kv_threads = 256;
+std::atomic<int> g_kv_threads{256};
+
+int check_threads(int threads)
+{
+    if (threads < 32 || threads > 256 || threads % 32 != 0) return fail("kv transfer: %d threads per CTA not in [32, 256] or not a multiple of 32", threads);
+    return 0;
+}
 
 }  // namespace
 
 extern "C" {
 
-// Threads per CTA of the transfer kernel (32 .. 256, a multiple of 32; default 256) for the whole process. Below the default
-// the copy goes through registers and takes no shared memory, so that its CTAs fit beside a GEMM's. A transfer
-// that runs beside a GEMM is best spread thin: one small CTA on every SM slows every GEMM CTA a little, a few large
-// CTAs slow a few GEMM CTAs a lot, and the GEMM ends with its slowest CTA.
+// Threads per CTA of the register form (32 .. 256, a multiple of 32; default 256) where a call names none, for the whole
+// process. A transfer that runs beside a GEMM is best spread thin: one small CTA on every SM slows every GEMM CTA a
+// little, a few large CTAs slow a few GEMM CTAs a lot, and the GEMM ends with its slowest CTA.
 int slime_kv_tune(int threads)
 {
-    if (threads < 32 || threads > 256 || threads % 32 != 0) return fail("kv transfer: %d threads per CTA not in [32, 256] or not a multiple of 32", threads);
+    if (check_threads(threads)) return -1;
     g_kv_threads = threads;
     return 0;
 }
@@ -281,6 +288,23 @@ int slime_kv_transfer(unsigned long long tok_k, unsigned long long tok_v, unsign
                       unsigned long long page_blocks, int to_paged, void* done_flag, unsigned long long done_value,
                       unsigned int* block_counter, int max_blocks, void* status, void* stream)
 {
+    return slime_kv_transfer_form(tok_k, tok_v, page_k, page_v, tok_off, blk, ntok, n_tasks, page_tokens, row_bytes, tok_rows, page_blocks,
+                                  to_paged, done_flag, done_value, block_counter, max_blocks, SLIME_KV_AUTO, 0, status, stream);
+}
+
+// The same with the form and (register form) the threads per CTA of this call; threads 0: what slime_kv_tune set.
+// SLIME_KV_AUTO takes bulk copies for pages of 16 KB and more, unless the process has tuned the register form's CTAs. Bulk copies
+// hold 192 KB of shared memory per CTA, so they never share an SM with a GEMM's CTA: for a transfer under compute
+// the caller names SLIME_KV_REGISTERS.
+int slime_kv_transfer_form(unsigned long long tok_k, unsigned long long tok_v, unsigned long long page_k,
+                           unsigned long long page_v, const int* tok_off, const int* blk, const int* ntok, int n_tasks,
+                           int page_tokens, unsigned long long row_bytes, unsigned long long tok_rows,
+                           unsigned long long page_blocks, int to_paged, void* done_flag, unsigned long long done_value,
+                           unsigned int* block_counter, int max_blocks, int form, int threads, void* status, void* stream)
+{
+    if (form < SLIME_KV_AUTO || form > SLIME_KV_BULK) return fail("kv transfer: unknown form %d", form);
+    if (threads == 0) threads = g_kv_threads;
+    else if (check_threads(threads)) return -1;
     if (n_tasks < 0 || page_tokens <= 0) return fail("kv transfer: bad task count or page size");
     if (row_bytes == 0 || row_bytes % 16 != 0) return fail("kv transfer: row_bytes (%llu) must be a positive multiple of 16", row_bytes);
     if (((tok_k | tok_v | page_k | page_v) & 15) != 0) return fail("kv transfer: plane addresses must be 16-byte aligned");
@@ -294,7 +318,7 @@ int slime_kv_transfer(unsigned long long tok_k, unsigned long long tok_v, unsign
     a.done_value    = done_value;
     a.block_counter = block_counter;
     a.status        = static_cast<KernelStatus*>(status);
-    if (g_kv_threads == 256 && static_cast<unsigned long long>(page_tokens) * row_bytes >= kKvChunk) {
+    if (form == SLIME_KV_BULK || (form == SLIME_KV_AUTO && threads == 256 && static_cast<unsigned long long>(page_tokens) * row_bytes >= kKvChunk)) {
         const unsigned long long page  = static_cast<unsigned long long>(page_tokens) * row_bytes;
         const long long          items = 2ll * n_tasks * static_cast<long long>((page + kKvChunk - 1) / kKvChunk);
         long long                ctas  = max_blocks > 0 ? max_blocks : sm_count();
@@ -308,14 +332,14 @@ int slime_kv_transfer(unsigned long long tok_k, unsigned long long tok_v, unsign
     }
     const unsigned long long slices = (static_cast<unsigned long long>(page_tokens) * row_bytes / 16 + kSliceSpan - 1) / kSliceSpan;
     if (slices > 0x7fffffffull) return fail("kv transfer: a page of %d rows of %llu bytes is too large", page_tokens, row_bytes);
-    const long long warps = g_kv_threads / 32;
+    const long long warps = threads / 32;
     long long       grid  = (2ll * n_tasks * static_cast<long long>(slices) + warps - 1) / warps;
     const long long cap = max_blocks > 0 ? max_blocks : sm_count() * 4;
     if (grid > cap) grid = cap;
     if (grid < 1) grid = 1;
     static bool carveout[64] = {false};  // runs beside the prefill GEMMs: see prefer_max_shared_carveout
     SLIME_CUDA_OK(prefer_max_shared_carveout(kv_transfer_kernel, carveout));
-    kv_transfer_kernel<<<static_cast<int>(grid), g_kv_threads, 0, static_cast<cudaStream_t>(stream)>>>(a);
+    kv_transfer_kernel<<<static_cast<int>(grid), threads, 0, static_cast<cudaStream_t>(stream)>>>(a);
     SLIME_CUDA_OK(cudaGetLastError());
     return 0;
 }

@@ -82,12 +82,10 @@ class PrefillSender:
 
     def __init__(self, shape: KVShape, dst_cache: PagedKVCache, max_tokens: int, comm_blocks: int = 32, comm_threads: int = 256):
         self.shape, self.dst, self.max_tokens = shape, dst_cache, max_tokens
-        if comm_threads != 256:
-            kv.tune(comm_threads)
         self.kv_stage = torch.empty((shape.layers, 2, max_tokens, shape.row), dtype=shape.dtype, device="cuda")
         self.comm_stream = torch.cuda.Stream(priority=-1)  # transfer CTAs should be placed ahead of the next GEMM's
         self.counter = torch.zeros(1, dtype=torch.int32, device="cuda")
-        self.comm_blocks = comm_blocks
+        self.comm_blocks, self.comm_threads = comm_blocks, comm_threads
         self.step = 0
 
     def plan(self, prompt_lens, dst_blocks):
@@ -98,14 +96,16 @@ class PrefillSender:
         self.step += 1
         return self.tasks
 
-    def send_layer(self, layer: int, stream=None) -> None:
+    def send_layer(self, layer: int, stream=None, form: str = "auto") -> None:
+        """Push one layer's pages; ``form`` as in :func:`kv.kv_move`, for the sender's own CTAs."""
         tok_off, blk, ntok = self.tasks
         s = self.shape
         kv.kv_move(self.kv_stage[layer, 0].data_ptr(), self.kv_stage[layer, 1].data_ptr(),
                    self.dst.plane_addr(layer, 0), self.dst.plane_addr(layer, 1), tok_off, blk, ntok,
                    page_tokens=s.page_tokens, row_bytes=s.row_bytes, tok_rows=self.max_tokens,
                    page_blocks=self.dst.num_blocks, to_paged=True, done_flag=self.dst.flag_addr(layer),
-                   done_value=self.step, counter=self.counter, max_blocks=self.comm_blocks, stream=stream)
+                   done_value=self.step, counter=self.counter, max_blocks=self.comm_blocks, stream=stream, form=form,
+                   threads=self.comm_threads)
 
     def run_prefill_with_transfer(self, hidden: torch.Tensor, weights: list[torch.Tensor], overlap: bool = True):
         """Synthetic prefill: one [tokens, d] x [d, d] GEMM per layer; layer l's KV goes out while l+1 computes.
@@ -122,7 +122,7 @@ class PrefillSender:
             if overlap:
                 self.comm_stream.wait_stream(main)
                 with torch.cuda.stream(self.comm_stream):
-                    self.send_layer(layer, self.comm_stream)
+                    self.send_layer(layer, self.comm_stream, form="registers")
             else:
                 self.send_layer(layer)
         if overlap:

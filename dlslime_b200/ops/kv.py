@@ -21,6 +21,9 @@ from ._common import default_status, ptr, stream_ptr
 
 _v, _i, _ull = ctypes.c_void_p, ctypes.c_int, ctypes.c_ulonglong
 _lib.declare("slime_kv_transfer", [_ull, _ull, _ull, _ull, _v, _v, _v, _i, _i, _ull, _ull, _ull, _i, _v, _ull, _v, _i, _v, _v])
+_lib.declare("slime_kv_transfer_form", [_ull, _ull, _ull, _ull, _v, _v, _v, _i, _i, _ull, _ull, _ull, _i, _v, _ull, _v, _i, _i, _i, _v, _v])
+
+_FORMS = {"auto": 0, "registers": 1, "bulk": 2}
 
 
 def build_page_tasks(prompt_lens, page_tokens: int, dst_blocks, src_starts=None, device="cuda"):
@@ -44,19 +47,23 @@ def build_page_tasks(prompt_lens, page_tokens: int, dst_blocks, src_starts=None,
 
 
 def tune(threads: int) -> None:
-    """Threads per CTA of the transfer kernel for the whole process (32 .. 256). With ``max_blocks`` = one CTA per SM and
-    64 threads a transfer that runs beside a GEMM is spread evenly over the SMs instead of slowing a few of them."""
+    """Threads per CTA of the register form for the whole process (32 .. 256), where a call names none. With ``max_blocks`` =
+    one CTA per SM and 64 threads a transfer that runs beside a GEMM is spread evenly over the SMs instead of slowing a few."""
     _lib.call("slime_kv_tune", int(threads))
 
 
 def kv_move(tok_k: int, tok_v: int, page_k: int, page_v: int, tok_off: torch.Tensor, blk: torch.Tensor,
             ntok: torch.Tensor | None, *, page_tokens: int, row_bytes: int, tok_rows: int, page_blocks: int,
             to_paged: bool = True, done_flag: int | None = None, done_value: int = 0, counter: torch.Tensor | None = None,
-            max_blocks: int = 0, stream=None) -> None:
-    """Launch one K+V page move (addresses are integers; the paged side may be a peer mapping)."""
-    _lib.call("slime_kv_transfer", tok_k, tok_v, page_k, page_v, ptr(tok_off), ptr(blk), ptr(ntok), tok_off.numel(),
+            max_blocks: int = 0, stream=None, form: str = "auto", threads: int = 0) -> None:
+    """Launch one K+V page move (addresses are integers; the paged side may be a peer mapping).
+
+    ``form``: ``"registers"`` (CTAs of ``threads`` threads without shared memory, which fit beside a GEMM's), ``"bulk"`` (the
+    bulk-copy engine, 192 KB of shared memory per CTA) or ``"auto"``: bulk copies for pages of 16 KB and more, unless
+    ``threads`` or :func:`tune` asks for other CTAs than the register form's 256 threads."""
+    _lib.call("slime_kv_transfer_form", tok_k, tok_v, page_k, page_v, ptr(tok_off), ptr(blk), ptr(ntok), tok_off.numel(),
               page_tokens, row_bytes, tok_rows, page_blocks, int(to_paged), done_flag, done_value, ptr(counter),
-              max_blocks, default_status().dev_ptr, stream_ptr(stream))
+              max_blocks, _FORMS[form], int(threads), default_status().dev_ptr, stream_ptr(stream))
 
 
 def kv_pack(tokens_kv: torch.Tensor, paged_kv: torch.Tensor, tok_off, blk, ntok=None) -> None:

@@ -113,3 +113,25 @@ def test_page_sizes_that_are_no_multiple_of_a_slice(page, row, lens, threads):
             back.fill_(4.0)
     finally:
         kv.tune(256)
+
+
+@pytest.mark.parametrize("form,threads", [("registers", 0), ("registers", 96), ("bulk", 0), ("auto", 64)])
+@pytest.mark.parametrize("page,row,lens", [(1, 8, [5, 1]), (64, 256, [63, 65, 640]), (64, 4104, [64, 129, 1])])
+def test_every_form_moves_the_same_bytes(page, row, lens, form, threads):
+    """The form a call names, for pages below, at and above one bulk chunk (16 B, 32 KB, 513 KB), with short last pages."""
+    from dlslime_b200.ops import kv
+    from dlslime_b200.ops._common import default_status
+
+    (tok_off, blk, ntok), _, blocks = _setup(lens, page, row)
+    total, rb = sum(lens), row * 2
+    src = torch.randn(2, total, row, device="cuda").to(torch.bfloat16)
+    paged = torch.full((2, blocks, page, row), 3.0, device="cuda", dtype=torch.bfloat16)
+    expect, back = paged.clone(), torch.full_like(src, 4.0)
+    for t, b, n in zip(tok_off.tolist(), blk.tolist(), ntok.tolist()):
+        expect[:, b, :n] = src[:, t:t + n]
+    for to_paged, tok in ((True, src), (False, back)):
+        kv.kv_move(tok[0].data_ptr(), tok[1].data_ptr(), paged[0].data_ptr(), paged[1].data_ptr(), tok_off, blk, ntok, page_tokens=page,
+                   row_bytes=rb, tok_rows=total, page_blocks=blocks, to_paged=to_paged, max_blocks=5, form=form, threads=threads)
+    torch.cuda.synchronize()
+    default_status().check()
+    assert torch.equal(paged, expect) and torch.equal(back, src)
