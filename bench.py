@@ -445,9 +445,9 @@ def run_ours(args, rank, world, local):
 
     # phase breakdown (one extra instrumented pass; not part of the reported value)
     dev_x, dev_lg, out = h.dev_x, h.dev_lg, h.out
-    evs = [torch.cuda.Event(enable_timing=True) for _ in range(7)]
+    phases = layer.phases(dev_x[0], dev_lg[0], out)
+    evs = [torch.cuda.Event(enable_timing=True) for _ in range(len(phases) + 1)]
     sync_all(world)
-    e = None  # device-resident step counter, as in the timed loops
     # keep the GPU busy for ~1 ms first, so that the launches below are queued ahead of their execution and the short
     # phases are not measured as host launch latency
     try:
@@ -455,26 +455,16 @@ def run_ours(args, rank, world, local):
     except Exception:
         torch.empty(512 << 20, dtype=torch.uint8, device="cuda").fill_(1)
     evs[0].record()
-    layer.step_route(dev_lg[0], T, e)
-    evs[1].record()
-    layer.step_dispatch(dev_x[0], e)
-    evs[2].record()
-    layer.step_recv(T, e)
-    evs[3].record()
-    layer.step_gate_up()
-    evs[4].record()
-    layer.step_down()
-    evs[5].record()
-    layer.step_combine(out, T, e)
-    evs[6].record()
+    for (_, launch), ev in zip(phases, evs[1:]):
+        launch()
+        ev.record()
     sync_all(world)
-    names = ["route", "dispatch_quant_push", "recv_wait_dequant", "gate_up_swiglu_gemm", "down_gemm_combine_push", "combine_wait_reduce"]
-    breakdown = {n: round(max_over_ranks(evs[i].elapsed_time(evs[i + 1]) * 1e3, world), 1) for i, n in enumerate(names)}
+    breakdown = {n: round(max_over_ranks(evs[i].elapsed_time(evs[i + 1]) * 1e3, world), 1) for i, (n, _) in enumerate(phases)}
     after()
 
     res.update({
         "breakdown_us": dict(breakdown, note="one extra pass with the phases run one after the other, whatever the timed loop does"),
-        "launches": (18 if tbo is not None else 8 if layer.streamed else 5 if layer.world == 1 and not args.fuse_dequant else 6) * args.steps, "cuda_graph": graph is not None, "overlap": tbo is not None,
+        "launches": (18 if tbo is not None else 8 if layer.streamed else len(phases)) * args.steps, "cuda_graph": graph is not None, "overlap": tbo is not None,
         "weights_gb": (layer.w_gate_up.numel() + layer.w_down.numel()) * 2 / 1e9,
         "notes": {"dequant": "in the gate/up GEMM's A-tile loader" if args.fuse_dequant else "in dispatch (one rank)" if layer.world == 1 and tbo is None and not layer.streamed else "separate pass",
                   "phases": "dispatch, receive and gate/up GEMM at the same time (per-expert arrival words)" if layer.streamed else "one after the other",

@@ -289,23 +289,27 @@ class ExpertParallelMoE:
         """x [T, hidden] bf16, router logits [T, num_experts] fp32 -> [T, hidden] bf16."""
         if self.streamed:
             return self.forward_streamed(x, logits, out)
-        T = x.shape[0]
         if out is None:
             out = torch.empty_like(x)
-        # epoch=None: the step counter lives on the device, so this sequence of launches is graph-capturable
-        self.step_route(logits, T, None)
-        if self.world == 1 and not self.fuse_dequant and not self.thin_waits and self.buf.trace is None:
-            # one rank: no row crosses a wire, so dispatch writes what the receive would (the trace counts both kernels)
-            self.buf.dispatch_expand(x, self.xd, None)
-            self.step_gate_up(chained=1)
-            self.step_down(chained=2)  # the row groups are dispatch's, two kernels back
-        else:
-            self.step_dispatch(x, None)
-            self.step_experts(T, None)
-        self.step_combine(out, T, None)
+        for _, launch in self.phases(x, logits, out):
+            launch()
         return out
 
     __call__ = forward
+
+    def phases(self, x: torch.Tensor, logits: torch.Tensor, out: torch.Tensor) -> list:
+        """The launches of one step with its phases one after the other, as ``(name, launch)`` in their order."""
+        T = x.shape[0]
+        # epoch=None: the step counter lives on the device, so this sequence of launches is graph-capturable
+        route = ("route", lambda: self.step_route(logits, T, None))
+        combine = ("combine_wait_reduce", lambda: self.step_combine(out, T, None))
+        if self.world == 1 and not self.fuse_dequant and not self.thin_waits and self.buf.trace is None:
+            # one rank: no row crosses a wire, so dispatch writes what the receive would (the trace counts both kernels);
+            # the down projection's row groups are dispatch's, two kernels back
+            return [route, ("dispatch_quant_expand", lambda: self.buf.dispatch_expand(x, self.xd, None)),
+                    ("gate_up_swiglu_gemm", lambda: self.step_gate_up(chained=1)), ("down_gemm_combine_push", lambda: self.step_down(chained=2)), combine]
+        return [route, ("dispatch_quant_push", lambda: self.step_dispatch(x, None)), ("recv_wait_dequant", lambda: self.step_recv(T, None)),
+                ("gate_up_swiglu_gemm", self.step_gate_up), ("down_gemm_combine_push", self.step_down), combine]
 
     def capture(self, x: torch.Tensor, logits: torch.Tensor, out: torch.Tensor) -> "torch.cuda.CUDAGraph":
         """Capture one forward on fixed buffers into a CUDA graph (decode-size steps are launch-bound).

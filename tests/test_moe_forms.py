@@ -80,3 +80,28 @@ def test_products_of_few_tiles_follow_the_launchers_rule(monkeypatch, clusters, 
     monkeypatch.setattr(gemm._lib, "call", lambda name, *a: clusters if name == "slime_gemm_bf16_clusters" else calls.append(name))
     gemm.gemm_bf16(torch.empty(m, k, dtype=torch.bfloat16), torch.empty(2048, k, dtype=torch.bfloat16))
     assert calls == [entry]
+
+
+@pytest.mark.parametrize("world,fuse,thin,trace,names", [
+    (1, False, False, None, ["route", "dispatch_quant_expand", "gate_up_swiglu_gemm", "down_gemm_combine_push", "combine_wait_reduce"]),
+    (1, True, False, None, ["route", "dispatch_quant_push", "recv_wait_dequant", "gate_up_swiglu_gemm", "down_gemm_combine_push", "combine_wait_reduce"]),
+    (1, False, True, None, ["route", "dispatch_quant_push", "recv_wait_dequant", "gate_up_swiglu_gemm", "down_gemm_combine_push", "combine_wait_reduce"]),
+    (1, False, False, 7, ["route", "dispatch_quant_push", "recv_wait_dequant", "gate_up_swiglu_gemm", "down_gemm_combine_push", "combine_wait_reduce"]),
+    (2, False, False, None, ["route", "dispatch_quant_push", "recv_wait_dequant", "gate_up_swiglu_gemm", "down_gemm_combine_push", "combine_wait_reduce"]),
+])
+def test_a_step_runs_the_phases_it_reports(world, fuse, thin, trace, names):
+    """forward() launches exactly what phases() names (bench.py times those one by one): one rank expands in dispatch, unless
+    the receive kernel is needed."""
+    import torch
+
+    ran = []
+    layer = ExpertParallelMoE.__new__(ExpertParallelMoE)
+    layer.world, layer.fuse_dequant, layer.thin_waits, layer.streamed, layer.xd = world, fuse, thin, False, None
+    layer.buf = type("B", (), {"trace": trace, "dispatch_expand": lambda self, *a: ran.append("dispatch_quant_expand")})()
+    for attr, name in (("step_route", "route"), ("step_dispatch", "dispatch_quant_push"), ("step_recv", "recv_wait_dequant"),
+                       ("step_gate_up", "gate_up_swiglu_gemm"), ("step_down", "down_gemm_combine_push"), ("step_combine", "combine_wait_reduce")):
+        setattr(layer, attr, lambda *a, _n=name, **k: ran.append(_n))
+    x = torch.zeros(3, 8)
+    assert [n for n, _ in layer.phases(x, x, x)] == names
+    layer.forward(x, x)
+    assert ran == names
