@@ -279,3 +279,28 @@ def test_dispatch_expand_writes_what_dispatch_and_receive_do(tokens, hidden, ldx
         got[form] = (buf.group_offsets.clone(), buf.recv_info[:rows][order].clone(), y[:rows][order].clone())
     for a, b in zip(*got.values()):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("tokens,form", [(300, (False, 0, 0, 192)), (400, ("swap", 0, 0, 0)), (640, (False, 0, 0, 0)), (2200, (True, 0, 0, 0))])
+def test_one_rank_layer_in_every_form_of_its_expert_gemms(tokens, form):
+    """150, 200, 320 and 1100 rows per expert: the layer's own choices above the decode sizes, in the chain of launches that one rank
+    makes, over steps whose routing changes (the last one leaves half of the experts empty), against the oracle."""
+    from dlslime_b200.models.moe import ExpertParallelMoE, MoEConfig, expert_gemm_form, init_expert_weights, ref_moe_forward
+
+    cfg = MoEConfig(num_experts=8, topk=4, hidden=1024, intermediate=256)
+    assert expert_gemm_form(tokens * cfg.topk / cfg.num_experts, {}) == form
+    w = init_expert_weights(cfg, range(cfg.num_experts), "cuda", seed=5)
+    layer = ExpertParallelMoE(cfg, tokens, weights=w)
+    gen = torch.Generator(device="cuda").manual_seed(tokens)
+    for step in range(4):
+        x = torch.randn((tokens, cfg.hidden), generator=gen, device="cuda").to(torch.bfloat16)
+        lg = torch.randn((tokens, cfg.num_experts), generator=gen, device="cuda")
+        if step == 3:
+            lg[:, ::2] += 20.0
+        out = layer(x, lg)
+        torch.cuda.synchronize()
+        layer.buf.status.check()
+        ref, _, _ = ref_moe_forward(cfg, x, lg, *w)
+        err = (out.float() - ref.float()).abs()
+        # the roundings of the bf16 result and of the bf16 values it is summed from
+        assert (err <= ref.float().abs() * 2 ** -6 + ref.float().abs().mean() * 2 ** -5).all(), f"step {step}"

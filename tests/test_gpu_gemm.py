@@ -302,3 +302,41 @@ def test_gemm_bf16_few_tiles_share_k(m, n, k):
     default_status().check()
     _check(out[:m], a.float() @ b.float().t(), k)
     assert (out[m] == 7.0).all()
+
+
+@pytest.mark.parametrize("groups", [7, 256, 257, 300])
+def test_grouped_gemm_weights_on_m_chained(groups):
+    """Launches chained to the one in front: the second product fetches its first weights early (K of two blocks, less than the
+    ring; up to 256 groups, whose prefix fits in shared memory) and reads rows that the launch in front of it writes. New
+    rows every time, so that rows of an earlier pass would show; bit for bit what ordinary launches give."""
+    from dlslime_b200.ops import gemm
+    from dlslime_b200.ops._common import default_status
+
+    gen = torch.Generator(device="cuda").manual_seed(groups)
+    sizes = torch.randint(0, 70 if groups == 7 else 5, (groups,), generator=gen, device="cuda")
+    offs = torch.cat([torch.zeros(1, dtype=torch.int64, device="cuda"), sizes.cumsum(0)]).to(torch.int32)
+    total, mid, n = int(offs[-1]), 128, 160
+    w1 = (torch.randn((groups, 2 * mid, 256), generator=gen, device="cuda") * 0.1).to(torch.bfloat16)
+    w2 = (torch.randn((groups, n, mid), generator=gen, device="cuda") * 0.1).to(torch.bfloat16)
+    h, out = torch.empty((total, mid), device="cuda", dtype=torch.bfloat16), torch.empty((total, n), device="cuda", dtype=torch.bfloat16)
+    xs = [torch.randn((total, 256), generator=gen, device="cuda").to(torch.bfloat16) for _ in range(6)]
+    want = []
+    for x in xs:
+        gemm.grouped_gemm_bf16(x, w1, offs, out=h, epilogue=gemm.EPI_SWIGLU, tile_tokens=64)
+        want.append(gemm.grouped_gemm_bf16(h, w2, offs, tile_tokens=64))
+    torch.cuda.synchronize()
+    got = []
+    for x in xs:
+        gemm.grouped_gemm_bf16(x, w1, offs, out=h, epilogue=gemm.EPI_SWIGLU, tile_tokens=64, chained=1)
+        gemm.grouped_gemm_bf16(h, w2, offs, out=out, tile_tokens=64, chained=2)
+        got.append(out.clone())
+    torch.cuda.synchronize()
+    default_status().check()
+    for a, b in zip(got, want):
+        assert torch.equal(a, b)
+    x = xs[0].float()
+    for gi in (0, groups // 2, groups - 1):
+        r = slice(int(offs[gi]), int(offs[gi + 1]))
+        if r.stop > r.start:
+            g = (torch.nn.functional.silu(x[r] @ w1[gi, :mid].float().t()) * (x[r] @ w1[gi, mid:].float().t())).to(torch.bfloat16).float()
+            _check(want[0][r], g @ w2[gi].float().t(), mid)
