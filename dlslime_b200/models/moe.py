@@ -68,14 +68,16 @@ class ExpertGemmForm(NamedTuple):
     tile_tokens: int  # single CTAs, weights on the M side: most rows of a group per tile (0 = tokens on the M side)
 
 
-def expert_gemm_form(rows: float, env=None) -> ExpertGemmForm:
-    """The form for experts that expect ``rows`` rows each in a step.
+def expert_gemm_form(rows: float, depth: int, env=None) -> ExpertGemmForm:
+    """The form for experts that expect ``rows`` rows each in a step; ``depth`` is the smaller K of the two products, the smaller
+    one of hidden and intermediate width.
 
-    Measured at hidden 7168, intermediate 2048 on one rank, whole steps run back to back (other widths and more ranks take the
-    same lines). Below ``gemm.WT_MAX_ROWS`` rows the weights go on the M side of single CTAs (:func:`gemm.pick_tile_tokens`), from there to
-    ``gemm.SWAP_MAX_ROWS`` on the M side of CTA pairs. Then come 128-row tiles, and from 1024 rows pairs, whose larger tiles waste
-    little there: 2815 us a step against 2860 on single CTAs with 32 x 1024 rows, but 3775 against 3300 with 64 x 512 and 3085
-    against 2744 with 64 x 384.
+    Below ``gemm.WT_MAX_ROWS`` rows the weights go on the M side of single CTAs (:func:`gemm.pick_tile_tokens`), from there to
+    ``gemm.SWAP_MAX_ROWS`` on the M side of CTA pairs if the products are deep enough to hide that kernel's epilogue, which turns every
+    accumulator around through shared memory. One-rank steps, swapped pairs against 128-row tiles: 64 experts x 200 rows,
+    hidden 7168, intermediate 2048 1252 against 1569 us, 7168 x 1536 1099 / 1200, 4096 x 2048 738 / 877, 2048 x 2048 448 / 510, but 7168 x
+    1024 897 / 838, 2048 x 768 279 / 258, and 256 experts of 1024 x 256 451 / 300. Then come 128-row tiles, and from
+    1024 rows CTA pairs.
 
     The environment overrides the rule: SLIME_EP_PAIR_GEMM=0|1|wide|swap the kind; SLIME_EP_TILE_N, SLIME_EP_TILE_M=0|64 and
     SLIME_EP_TILE_TOKENS=0|64|128|192 the tiles of the single-CTA forms, so none of them goes with "swap" unless that is forced.
@@ -90,7 +92,7 @@ def expert_gemm_form(rows: float, env=None) -> ExpertGemmForm:
     tiles_given = bool(tile_n) or tile_m is not None or tile_tokens is not None
     if kind is not None:
         pair = {"0": False, "1": True}.get(kind, kind)
-    elif gemm.WT_MAX_ROWS <= rows < gemm.SWAP_MAX_ROWS and not tiles_given:
+    elif gemm.WT_MAX_ROWS <= rows < gemm.SWAP_MAX_ROWS and depth >= 1536 and not tiles_given:
         pair = "swap"
     else:
         pair = rows >= 1024
@@ -129,7 +131,7 @@ class ExpertParallelMoE:
         # words of the gated GEMM's dynamic tile scheduler (SLIME_EP_STATIC_TILES=1: every gridDim-th tile instead)
         self._tile_counter = None if os.environ.get("SLIME_EP_STATIC_TILES") == "1" else torch.zeros(2, dtype=torch.int32, device=dev)
         # pair_gemm, tile_n_*, tile_m, tile_tokens: see expert_gemm_form; autotune() measures and sets pair_gemm
-        form = expert_gemm_form(max_tokens * cfg.topk * self.world / max(1, cfg.num_experts))
+        form = expert_gemm_form(max_tokens * cfg.topk * self.world / max(1, cfg.num_experts), min(cfg.hidden, cfg.intermediate))
         self._default_pair_gemm = self.pair_gemm = form.pair
         self.tile_n_gate_up = self.tile_n_down = form.tile_n
         self.tile_m, self.tile_tokens = form.tile_m, form.tile_tokens

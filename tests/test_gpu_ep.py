@@ -281,14 +281,14 @@ def test_dispatch_expand_writes_what_dispatch_and_receive_do(tokens, hidden, ldx
         assert torch.equal(a, b)
 
 
-@pytest.mark.parametrize("tokens,form", [(300, (False, 0, 0, 192)), (400, ("swap", 0, 0, 0)), (640, (False, 0, 0, 0)), (2200, (True, 0, 0, 0))])
-def test_one_rank_layer_in_every_form_of_its_expert_gemms(tokens, form):
-    """150, 200, 320 and 1100 rows per expert: the layer's own choices above the decode sizes, in the chain of launches that one rank
-    makes, over steps whose routing changes (the last one leaves half of the experts empty), against the oracle."""
+@pytest.mark.parametrize("tokens,hidden,inter,form", [(300, 1024, 256, (False, 0, 0, 192)), (400, 2048, 1536, ("swap", 0, 0, 0)),
+                                                      (400, 1024, 256, (False, 0, 0, 0)), (2200, 1024, 256, (True, 0, 0, 0))])
+def test_one_rank_layer_in_every_form_of_its_expert_gemms(tokens, hidden, inter, form):
+    """150, 200 and 1100 rows per expert: the layer's own choices above the decode sizes, in the chain of launches that one rank makes, over steps whose routing changes (the last one leaves half of the experts empty), against the oracle."""
     from dlslime_b200.models.moe import ExpertParallelMoE, MoEConfig, expert_gemm_form, init_expert_weights, ref_moe_forward
 
-    cfg = MoEConfig(num_experts=8, topk=4, hidden=1024, intermediate=256)
-    assert expert_gemm_form(tokens * cfg.topk / cfg.num_experts, {}) == form
+    cfg = MoEConfig(num_experts=8, topk=4, hidden=hidden, intermediate=inter)
+    assert expert_gemm_form(tokens * cfg.topk / cfg.num_experts, min(hidden, inter), {}) == form
     w = init_expert_weights(cfg, range(cfg.num_experts), "cuda", seed=5)
     layer = ExpertParallelMoE(cfg, tokens, weights=w)
     gen = torch.Generator(device="cuda").manual_seed(tokens)

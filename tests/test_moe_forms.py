@@ -3,34 +3,41 @@ import pytest
 
 from dlslime_b200.models.moe import ExpertGemmForm, ExpertParallelMoE, expert_gemm_form
 
-RULE = {1: ExpertGemmForm(False, 0, 64, 64), 32: ExpertGemmForm(False, 0, 64, 64), 64: ExpertGemmForm(False, 0, 0, 128),
-        128: ExpertGemmForm(False, 0, 0, 192), 175.9: ExpertGemmForm(False, 0, 0, 192), 176: ExpertGemmForm("swap", 0, 0, 0),
-        200: ExpertGemmForm("swap", 0, 0, 0), 300: ExpertGemmForm("swap", 0, 0, 0), 320: ExpertGemmForm(False, 0, 0, 0),
-        500: ExpertGemmForm(False, 0, 0, 0), 1023: ExpertGemmForm(False, 0, 0, 0), 1024: ExpertGemmForm(True, 0, 0, 0)}
+ROWS = {1: ExpertGemmForm(False, 0, 64, 64), 32: ExpertGemmForm(False, 0, 64, 64), 64: ExpertGemmForm(False, 0, 0, 128),
+        128: ExpertGemmForm(False, 0, 0, 192), 175.9: ExpertGemmForm(False, 0, 0, 192), 320: ExpertGemmForm(False, 0, 0, 0),
+        500: ExpertGemmForm(False, 0, 0, 0), 1023: ExpertGemmForm(False, 0, 0, 0), 1024: ExpertGemmForm(True, 0, 0, 0), 4096: ExpertGemmForm(True, 0, 0, 0)}
 
 
-@pytest.mark.parametrize("rows,form", RULE.items())
-def test_rule_by_rows_per_expert(rows, form):
-    assert expert_gemm_form(rows, {}) == form
+@pytest.mark.parametrize("depth", [256, 1024, 2048, 7168])
+@pytest.mark.parametrize("rows,form", ROWS.items())
+def test_rule_by_rows_per_expert(rows, form, depth):
+    assert expert_gemm_form(rows, depth, {}) == form
+
+
+@pytest.mark.parametrize("depth,pair", [(256, False), (768, False), (1024, False), (1536, "swap"), (2048, "swap"), (7168, "swap")])
+@pytest.mark.parametrize("rows", [176, 200, 300, 319.9])
+def test_swapped_pairs_only_where_the_products_are_deep(rows, depth, pair):
+    """Narrow layers lose up to 1.5x on swapped pairs (256 experts of 1024 x 256, 256 rows each: 569 us a step against 348)."""
+    assert expert_gemm_form(rows, depth, {}) == ExpertGemmForm(pair, 0, 0, 0)
 
 
 @pytest.mark.parametrize("rows", [40, 200, 500])
 def test_overrides_are_taken_in_every_range(rows):
     """A tile override is one of the single-CTA forms, so it also holds where swapped pairs would be the default."""
-    assert expert_gemm_form(rows, {"SLIME_EP_TILE_TOKENS": "128"})[::3] == (False, 128)
-    assert expert_gemm_form(rows, {"SLIME_EP_TILE_N": "192"})[:2] == (False, 192)
-    assert expert_gemm_form(rows, {"SLIME_EP_TILE_N": "192"}).tile_tokens == 0
-    assert expert_gemm_form(rows, {"SLIME_EP_TILE_M": "64"})[:3] == (False, 0, 64)
-    assert expert_gemm_form(rows, {"SLIME_EP_PAIR_GEMM": "0"}).pair is False
-    assert expert_gemm_form(rows, {"SLIME_EP_PAIR_GEMM": "1"}).pair is True
-    assert expert_gemm_form(rows, {"SLIME_EP_PAIR_GEMM": "swap", "SLIME_EP_TILE_M": "0"}).pair == "swap"
+    assert expert_gemm_form(rows, 2048, {"SLIME_EP_TILE_TOKENS": "128"})[::3] == (False, 128)
+    assert expert_gemm_form(rows, 2048, {"SLIME_EP_TILE_N": "192"})[:2] == (False, 192)
+    assert expert_gemm_form(rows, 2048, {"SLIME_EP_TILE_N": "192"}).tile_tokens == 0
+    assert expert_gemm_form(rows, 2048, {"SLIME_EP_TILE_M": "64"})[:3] == (False, 0, 64)
+    assert expert_gemm_form(rows, 2048, {"SLIME_EP_PAIR_GEMM": "0"}).pair is False
+    assert expert_gemm_form(rows, 2048, {"SLIME_EP_PAIR_GEMM": "1"}).pair is True
+    assert expert_gemm_form(rows, 2048, {"SLIME_EP_PAIR_GEMM": "swap", "SLIME_EP_TILE_M": "0"}).pair == "swap"
 
 
 class _Timed(ExpertParallelMoE):
     """The layer without a GPU: a step takes what the table says for the form that is set."""
 
     def __init__(self, rows, times):
-        form = expert_gemm_form(rows, {})
+        form = expert_gemm_form(rows, 2048, {})
         self._default_pair_gemm = self.pair_gemm = form.pair
         self.tile_tokens, self.fuse_dequant, self.streamed = form.tile_tokens, False, False
         self.times, self.timed = times, []
