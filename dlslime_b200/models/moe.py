@@ -76,8 +76,9 @@ def expert_gemm_form(rows: float, depth: int, env=None) -> ExpertGemmForm:
     ``gemm.SWAP_MAX_ROWS`` on the M side of CTA pairs if the products are deep enough to hide that kernel's epilogue, which turns every
     accumulator around through shared memory. One-rank steps, swapped pairs against 128-row tiles: 64 experts x 200 rows,
     hidden 7168, intermediate 2048 1252 against 1569 us, 7168 x 1536 1099 / 1200, 4096 x 2048 738 / 877, 2048 x 2048 448 / 510, but 7168 x
-    1024 897 / 838, 2048 x 768 279 / 258, and 256 experts of 1024 x 256 451 / 300. Then come 128-row tiles, and from
-    1024 rows CTA pairs.
+    1024 897 / 838, 2048 x 768 279 / 258, and 256 experts of 1024 x 256 451 / 300. Up to 512 rows come 128-row tiles, from there
+    CTA pairs: 64 x 512 rows of 7168 x 2048 2722 us against 3095 with row tiles, 32 x 700 1680 / 2035, 32 x 1000 2258 / 2727,
+    64 x 512 of 4096 x 2048 1597 / 1796, 32 x 512 of 4096 x 1024 492 / 563, 128 x 512 of 1024 x 256 315 / 305.
 
     The environment overrides the rule: SLIME_EP_PAIR_GEMM=0|1|wide|swap the kind; SLIME_EP_TILE_N, SLIME_EP_TILE_M=0|64 and
     SLIME_EP_TILE_TOKENS=0|64|128|192 the tiles of the single-CTA forms, so none of them goes with "swap" unless that is forced.
@@ -95,7 +96,7 @@ def expert_gemm_form(rows: float, depth: int, env=None) -> ExpertGemmForm:
     elif gemm.WT_MAX_ROWS <= rows < gemm.SWAP_MAX_ROWS and depth >= 1536 and not tiles_given:
         pair = "swap"
     else:
-        pair = rows >= 1024
+        pair = rows >= 512
     few_rows = 64 if rows + 3 * rows ** 0.5 <= 64 else 0
     free = not tile_n and tile_m is None
     return ExpertGemmForm(pair, tile_n, few_rows if tile_m is None else int(tile_m),

@@ -5,7 +5,7 @@ from dlslime_b200.models.moe import ExpertGemmForm, ExpertParallelMoE, expert_ge
 
 ROWS = {1: ExpertGemmForm(False, 0, 64, 64), 32: ExpertGemmForm(False, 0, 64, 64), 64: ExpertGemmForm(False, 0, 0, 128),
         128: ExpertGemmForm(False, 0, 0, 192), 175.9: ExpertGemmForm(False, 0, 0, 192), 320: ExpertGemmForm(False, 0, 0, 0),
-        500: ExpertGemmForm(False, 0, 0, 0), 1023: ExpertGemmForm(False, 0, 0, 0), 1024: ExpertGemmForm(True, 0, 0, 0), 4096: ExpertGemmForm(True, 0, 0, 0)}
+        500: ExpertGemmForm(False, 0, 0, 0), 512: ExpertGemmForm(True, 0, 0, 0), 1023: ExpertGemmForm(True, 0, 0, 0), 4096: ExpertGemmForm(True, 0, 0, 0)}
 
 
 @pytest.mark.parametrize("depth", [256, 1024, 2048, 7168])
