@@ -293,9 +293,9 @@ int slime_kv_transfer(unsigned long long tok_k, unsigned long long tok_v, unsign
 }
 
 // The same with the form and (register form) the threads per CTA of this call; threads 0: what slime_kv_tune set.
-// SLIME_KV_AUTO takes bulk copies for pages of 16 KB and more, unless the process has tuned the register form's CTAs. Bulk copies
-// hold 192 KB of shared memory per CTA, so they never share an SM with a GEMM's CTA: for a transfer under compute
-// the caller names SLIME_KV_REGISTERS.
+// SLIME_KV_AUTO takes bulk copies for pages of 16 KB and more, unless this call or the process asks for other CTAs than the
+// register form's 256 threads. Bulk copies hold 192 KB of shared memory per CTA, so they never share an SM with a GEMM's CTA: a
+// caller whose transfer runs under compute for long names SLIME_KV_REGISTERS.
 int slime_kv_transfer_form(unsigned long long tok_k, unsigned long long tok_v, unsigned long long page_k,
                            unsigned long long page_v, const int* tok_off, const int* blk, const int* ntok, int n_tasks,
                            int page_tokens, unsigned long long row_bytes, unsigned long long tok_rows,

@@ -50,10 +50,11 @@ def test_kv_transfer_refuses_forms_and_ctas_it_does_not_have(form, threads, say)
         _lib.call("slime_kv_transfer_form", A, A, B, B, OFFS, OFFS, None, 1, 64, 512, 64, 4, 1, None, 0, None, 0, form, threads, None, None)
 
 
+@pytest.mark.parametrize("rank,under_compute", [(0, "auto"), (1, "registers")])
 @pytest.mark.parametrize("threads", [256, 64])
-def test_prefill_transfer_under_compute_names_the_form_that_fits_beside_a_gemm(monkeypatch, threads):
-    """Under the GEMM chain the sender asks for CTAs without shared memory, by itself the push is left to the launcher's rule; both with
-    the sender's own CTAs, whatever other senders of the process have."""
+def test_prefill_transfer_under_compute_names_its_form(monkeypatch, threads, rank, under_compute):
+    """Under the GEMM chain a sender to another GPU asks for CTAs without shared memory; otherwise the form is left to the launcher's
+    rule. Always with the sender's own CTAs, whatever other senders of the process have."""
     import contextlib
 
     import torch
@@ -71,11 +72,12 @@ def test_prefill_transfer_under_compute_names_the_form_that_fits_beside_a_gemm(m
     monkeypatch.setattr(pd_kv.gemm, "gemm_bf16", lambda a, w, out=None: out)
     monkeypatch.setattr(pd_kv.kv, "kv_move", lambda *a, **k: moves.append((k["form"], k["threads"])))
     monkeypatch.setattr(pd_kv.kv, "tune", lambda t: moves.append(("tuned the process", t)))
-    cache = type("C", (), {"plane_addr": lambda self, *a: 0, "flag_addr": lambda self, layer: 0, "num_blocks": 4})()
+    cache = type("C", (), {"plane_addr": lambda self, *a: 0, "flag_addr": lambda self, layer: 0, "num_blocks": 4, "owner": 0,
+                           "heap": type("H", (), {"rank": rank})})()
     sender = pd_kv.PrefillSender(pd_kv.KVShape(layers=2), cache, max_tokens=64, comm_threads=threads)
     sender.tasks = (None, None, None)
     sender.send_layer(0)
     hidden = real_empty(64, 8)
     sender.run_prefill_with_transfer(hidden, [hidden], overlap=True)
     sender.run_prefill_with_transfer(hidden, [hidden], overlap=False)
-    assert moves == [("auto", threads), ("registers", threads), ("registers", threads), ("auto", threads), ("auto", threads)]
+    assert moves == [("auto", threads)] + 2 * [(under_compute, threads)] + 2 * [("auto", threads)]
