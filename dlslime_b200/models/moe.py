@@ -292,23 +292,35 @@ class ExpertParallelMoE:
         """x [T, hidden] bf16, router logits [T, num_experts] fp32 -> [T, hidden] bf16."""
         if self.streamed:
             return self.forward_streamed(x, logits, out)
+        T = x.shape[0]
         if out is None:
             out = torch.empty_like(x)
-        for _, launch in self.phases(x, logits, out):
-            launch()
+        # epoch=None: the step counter lives on the device, so this sequence of launches is graph-capturable
+        self.step_route(logits, T, None)
+        if self._expands_in_dispatch:
+            self.buf.dispatch_expand(x, self.xd, None)
+            self.step_gate_up(chained=1)
+            self.step_down(chained=2)  # the row groups are dispatch's, two kernels back
+        else:
+            self.step_dispatch(x, None)
+            self.step_experts(T, None)
+        self.step_combine(out, T, None)
         return out
 
     __call__ = forward
 
+    @property
+    def _expands_in_dispatch(self) -> bool:
+        """One rank: no row crosses a wire, so dispatch writes what the receive would (the trace counts both kernels)."""
+        return self.world == 1 and not self.fuse_dequant and not self.thin_waits and self.buf.trace is None
+
     def phases(self, x: torch.Tensor, logits: torch.Tensor, out: torch.Tensor) -> list:
-        """The launches of one step with its phases one after the other, as ``(name, launch)`` in their order."""
+        """The launches that :meth:`forward` makes with its phases one after the other, as ``(name, launch)`` in their order. (forward
+        does not go through this list: making it costs 3 us a step.)"""
         T = x.shape[0]
-        # epoch=None: the step counter lives on the device, so this sequence of launches is graph-capturable
         route = ("route", lambda: self.step_route(logits, T, None))
         combine = ("combine_wait_reduce", lambda: self.step_combine(out, T, None))
-        if self.world == 1 and not self.fuse_dequant and not self.thin_waits and self.buf.trace is None:
-            # one rank: no row crosses a wire, so dispatch writes what the receive would (the trace counts both kernels);
-            # the down projection's row groups are dispatch's, two kernels back
+        if self._expands_in_dispatch:
             return [route, ("dispatch_quant_expand", lambda: self.buf.dispatch_expand(x, self.xd, None)),
                     ("gate_up_swiglu_gemm", lambda: self.step_gate_up(chained=1)), ("down_gemm_combine_push", lambda: self.step_down(chained=2)), combine]
         return [route, ("dispatch_quant_push", lambda: self.step_dispatch(x, None)), ("recv_wait_dequant", lambda: self.step_recv(T, None)),

@@ -109,6 +109,10 @@ def test_a_step_runs_the_phases_it_reports(world, fuse, thin, trace, names):
                        ("step_gate_up", "gate_up_swiglu_gemm"), ("step_down", "down_gemm_combine_push"), ("step_combine", "combine_wait_reduce")):
         setattr(layer, attr, lambda *a, _n=name, **k: ran.append(_n))
     x = torch.zeros(3, 8)
-    assert [n for n, _ in layer.phases(x, x, x)] == names
+    phases = layer.phases(x, x, x)
+    assert [n for n, _ in phases] == names
     layer.forward(x, x)
     assert ran == names
+    for _, launch in phases:
+        launch()
+    assert ran == 2 * names
