@@ -40,7 +40,7 @@ class KVShape:
 
     @property
     def row_bytes(self) -> int:
-        return self.row * torch.empty((), dtype=self.dtype).element_size()
+        return self.row * self.dtype.itemsize
 
     @property
     def page_bytes(self) -> int:
