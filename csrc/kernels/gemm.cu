@@ -9,6 +9,8 @@
 #include "common/host_utils.h"
 #include "slime_cuda.h"
 
+#include <algorithm>
+
 using namespace slime;
 using namespace slime::gemm;
 
@@ -74,13 +76,16 @@ thread_local int g_w_prefetch = 0;  // and the distance of its weight prefetch i
 thread_local int g_tile_m     = 0;  // 64: row tiles of 64 with a five-stage ring (groups of a few dozen rows)
 
 // CTAs per tile for a product with fewer 128 x 256 tiles than a quarter of the SMs: as many (2, 4 or 8) as all run at the same
-// time, if that shortens each CTA's run by 14 K blocks, about what meeting twice and adding the sums costs. 1 = no split.
+// time, if that shortens each CTA's run by the K blocks that meeting twice and adding the sums cost: 14 for tiles of up to 64 rows,
+// 19 for 128, whose sums are twice as many (64 x 2048 x 1024, 14 blocks less: 9.4 -> 7.9 us; 128 x 2048 x 1024: 9.1 -> 10.6,
+// so not split; 128 x 2048 x 1536, 21 blocks less: 11.9 -> 10.9). 1 = no split.
 int pick_ksplit(int M, int N, int K)
 {
     static int  cached[64][3]  = {};
     static bool configured[64] = {};
     const long  tiles   = static_cast<long>((M + kBM - 1) / kBM) * ((N + kKsBN - 1) / kKsBN);
     const int   kblocks = (K + kBK - 1) / kBK;
+    const int   worth   = std::max(14, 9 + std::min(M, kBM) * 10 / kBM);
     if (4 * tiles > sm_count()) return 1;
     if (allow_dynamic_smem(gemm_bf16_ksplit_kernel, kKsSmem, configured) != cudaSuccess) {
         cudaGetLastError();
@@ -88,7 +93,7 @@ int pick_ksplit(int M, int N, int K)
     }
     int split = 1;
     for (int c : {2, 4, 8})
-        if (kblocks - kblocks / c >= 14 && tiles <= max_active_clusters(gemm_bf16_ksplit_kernel, c, kThreads, kKsSmem, cached)) split = c;
+        if (kblocks - kblocks / c >= worth && tiles <= max_active_clusters(gemm_bf16_ksplit_kernel, c, kThreads, kKsSmem, cached)) split = c;
     return split;
 }
 

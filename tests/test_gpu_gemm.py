@@ -340,3 +340,12 @@ def test_grouped_gemm_weights_on_m_chained(groups):
         if r.stop > r.start:
             g = (torch.nn.functional.silu(x[r] @ w1[gi, :mid].float().t()) * (x[r] @ w1[gi, mid:].float().t())).to(torch.bfloat16).float()
             _check(want[0][r], g @ w2[gi].float().t(), mid)
+
+
+@pytest.mark.parametrize("m,k,shared", [(64, 1024, True), (65, 1024, True), (128, 1024, False), (128, 1472, True), (300, 1472, True), (300, 1024, False), (16, 832, False)])
+def test_clusters_are_worth_more_k_blocks_for_taller_tiles(m, k, shared):
+    """The launcher shares a tile's K where that saves 14 K blocks per CTA, 19 for tiles of 128 rows, whose sums are twice as many."""
+    from dlslime_b200 import _lib
+
+    assert (_lib.call("slime_gemm_bf16_clusters", m, 2048, k) > 1) is shared
+    test_gemm_bf16_few_tiles_share_k(m, 2048, k)
