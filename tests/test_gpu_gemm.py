@@ -342,7 +342,7 @@ def test_grouped_gemm_weights_on_m_chained(groups):
             _check(want[0][r], g @ w2[gi].float().t(), mid)
 
 
-@pytest.mark.parametrize("m,k,shared", [(64, 1024, True), (65, 1024, True), (128, 1024, False), (128, 1472, True), (300, 1472, True), (300, 1024, False), (16, 832, False)])
+@pytest.mark.parametrize("m,k,shared", [(64, 1024, True), (65, 1024, True), (128, 1024, False), (128, 1472, True), (300, 1664, True), (300, 1472, False), (16, 832, False)])
 def test_clusters_are_worth_more_k_blocks_for_taller_tiles(m, k, shared):
     """The launcher shares a tile's K where that saves 14 K blocks per CTA, 19 for tiles of 128 rows, whose sums are twice as many."""
     from dlslime_b200 import _lib
