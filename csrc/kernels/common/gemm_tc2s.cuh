@@ -18,10 +18,10 @@
 // Tiles of a group: ceil(rows / 256) equal parts (rounded up to 16 tokens), part fastest, then the feature tile
 // (256 weight rows per pair: 256 output columns, or 128 for SwiGLU).
 //
-// Measured as whole one-rank steps (hidden 7168, intermediate 2048), run back to back at the power limit, against row tiles on single
-// CTAs: 128 experts x 192 rows 2640 against 3139 us, x 224 2890 / 3161, x 256 3555 / 3744, 64 x 384 2580 / 2600, x 512 3310 / 3200, 32 x 1024
-// 2870 / 2860. The layer takes it from 176 to 320 rows per expert; below, the tiles of gemm_wt.cuh hold a group as well and need no
-// partner. Loading only the token rows that exist, with boxes of 32 and 8 instead of one of 128, was slower (256 rows: 3850 -> 4209 us):
+// Measured as whole one-rank steps (hidden 7168, intermediate 2048), replayed from graphs in turn with row tiles on single CTAs: 128
+// experts x 192 rows 2397 against 3166 us, x 224 2602 / 3218, x 256 3405 / 3690, x 300 4075 / 4273, x 320 4307 / 4227. The layer takes it
+// from 176 to 320 rows per expert, and only where both products are at least 1536 deep: an accumulator takes as long to turn around
+// however short its main loop was (256 experts of 1024 x 256 with 256 rows: 569 against 348 us a step). Loading only the token rows that exist, with boxes of 32 and 8 instead of one of 128, was slower (256 rows: 3850 -> 4209 us):
 // more TMA operations cost more than the bytes they save.
 #pragma once
 

@@ -8,13 +8,13 @@
 //
 // What bounds such a launch, and why this shape: every weight byte is read from HBM once (6.9-7.0 TB/s for a bare TMA
 // stream with 96-128 KB in flight per SM), but it also has to get into the SM beside the tokens, at 64 bytes per clock, and at
-// full load the power limit holds the SM clock at 1.0-1.2 GHz. With tokens on the M side a group of 128 +- 11 rows is one or two
+// full load the power limit holds the SM clock at 1.1-1.4 GHz. With tokens on the M side a group of 128 +- 11 rows is one or two
 // 128-row tiles, so a 64-deep K block of 256 weight rows costs 48 KB per row tile, 70 KB on average, and 1.47 times the
 // rows that exist go through the tensor core. Here it costs 32 KB + 128 bytes per token, 50 KB, and the MMAs
-// are as wide as the group. Whole one-rank steps, hidden 7168, intermediate 2048, run back to back at the power limit, against
-// the row-tiled kernel: 256 experts x 128 rows 6090 -> 5020 us, 64 x 97 rows 1125 -> 1082 us, 32 x 32 rows 559 -> 514 us, 19 x 1
-// 354 -> 339 us; 128 experts x 160 rows 3510 -> 2798, x 192 rows 3541 -> 3321, x 256 rows 4126 -> 4952: there a group is two
-// parts whose accumulators leave no room for a second buffer, and the row tiles waste little.
+// are as wide as the group. Whole one-rank steps, hidden 7168, intermediate 2048, replayed from graphs in turn with the row-tiled
+// kernel in the same step: 128 experts x 128 rows 2426 -> 2183 us, x 160 rows 3009 -> 2341, x 192 rows 3166 -> 2970, x 256 rows
+// 3690 -> 4204: there a group is two parts whose accumulators leave no room for a second buffer, and the row tiles waste little.
+// When it came in: 64 x 97 rows 1125 -> 1082 us, 32 x 32 rows 559 -> 514 us, 19 x 1 354 -> 339 us.
 //
 // The accumulator is transposed: tensor-memory lanes are features, columns are tokens. Eight epilogue warps (two per lane
 // quadrant, taking 32-token chunks in turn) round to bf16, turn a 32-token x 128-feature block around in shared memory

@@ -10,13 +10,14 @@
 // source (pack, or prefill -> decode transfer when the paged side is a peer's cache);
 // otherwise the paged side is the source (unpack).
 //
-// One launch moves K and V of one layer for the whole batch: warps walk 4 KB slices of the (task, plane) pages.
+// One launch moves K and V of one layer for the whole batch, through registers (warps walk 4 KB slices of the (task, plane)
+// pages) or, for pages of 16 KB and more, through the bulk-copy engine (kv_bulk_kernel).
 // The last CTA to finish publishes `done_value` at `done_flag` (release, system scope), typically a per-layer
 // word in the decode rank's memory, so the consumer can start attention on layer l while
 // layer l+1 is still in flight.
 //
-// A transfer that runs beside the prefill GEMMs gets few CTAs (32 by default) without shared memory, so its rate is
-// the bytes that those CTAs keep in flight over the memory latency. Every warp has a slice being stored, the next one on
+// Register form. Its CTAs take no shared memory, so they fit beside a GEMM's, and a transfer that runs beside the prefill
+// GEMMs gets few of them (32 by default): its rate is the bytes that those keep in flight over the memory latency. Every warp has a slice being stored, the next one on
 // its way and the page header of the one after that, whatever the page size. (With one page per CTA at a time, its
 // header fetched when the CTA came to it, nothing was in flight between two pages: 30 MB per layer, 32 CTAs, 64-token pages of 512-byte
 // rows took 55 us a layer where this takes 42 us, and 4 KB pages left most of a CTA idle. With 148 CTAs it is 20 us,
@@ -152,9 +153,10 @@ __global__ void __launch_bounds__(256) kv_transfer_kernel(KvArgs a)
 // The same move through the bulk-copy engine, one warp per CTA: global -> shared bulk loads run ahead of the shared -> global
 // bulk stores by a ring of 192 KB, so that a CTA keeps more than the bytes of the register form in flight, without a break
 // between pages. The page headers of 32 chunks are resolved at a time, one per lane, and those of the
-// next 32 are on their way meanwhile. Five prompts, 32 KB pages, per layer: 32 CTAs 41 -> 35 us (54 GB/s read and written per SM,
-// of about 70 that an SM gets from HBM), 148 CTAs 18.7 -> 16.9 us; one layer of 16 prompts with 64 KB pages on all SMs 45 -> 41 us.
-// One thread issues about four chunks per microsecond, so 4 KB pages stay with the register form (12 us against 29).
+// next 32 are on their way meanwhile. Layers replayed back to back from a graph, register form -> this: five prompts, 32 KB pages
+// (30 MB) on 32 CTAs 43.6 -> 29.8 us, 31 GB/s in and 31 out per SM, on 148 CTAs 21.0 -> 19.2 us; 16 prompts, 64 KB pages (167 MB)
+// on 32 CTAs 199 -> 119 us, on 148 72.5 -> 63.4 us, 5.3 TB/s read and written. Which of an SM's two directions stops a CTA is not
+// known. Smaller chunks cost more issue than they carry: 8 KB pages take 44.1 us through registers, 45.6 here (32 CTAs).
 constexpr int kKvRingBytes = 192 * 1024;
 constexpr int kKvChunk     = 16 * 1024;
 constexpr int kKvSlots     = kKvRingBytes / kKvChunk;

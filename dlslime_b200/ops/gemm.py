@@ -86,10 +86,10 @@ def pick_tile_tokens(rows_per_group: float) -> int:
     """``tile_tokens`` of :func:`grouped_gemm_bf16` for groups that are expected to hold ``rows_per_group`` rows each (0 = the
     row-tiled forms are the faster ones): the smallest tile that holds a group three standard deviations above the mean, so
     that a group's weights enter an SM once, and the most stages for it (64 experts x 97 rows: 1082 us a step with tiles of
-    128, 1380 with 64, 1105 with 192). Between ``WT_MAX_ROWS``
-    and ``SWAP_MAX_ROWS`` rows the swapped pairs win, whose tiles hold 256 (128 experts: 160 rows 2430 us here, 2450 on swapped pairs,
-    3080 with row tiles; 192 rows 2950, 2640, 3140; 256 rows 4210, 3555, 3745), from there on the row tiles (64 experts x 384 rows:
-    2552-2612 us on swapped pairs, 2600 with row tiles; 512 rows 3310, 3200)."""
+    128, 1380 with 64, 1105 with 192). Between ``WT_MAX_ROWS`` and ``SWAP_MAX_ROWS`` rows the tiles of the swapped pairs hold a group
+    and these do not. Steps of 128 experts, hidden 7168, intermediate 2048, here / on swapped pairs / with row tiles: 160 rows 2341 / 2215 /
+    3009 us, 192 rows 2970 / 2397 / 3166, 256 rows 4204 / 3405 / 3690, 320 rows 4168 / 4307 / 4227; of 64 experts: 160 rows
+    1229 / 1183 / 1551, 320 rows 2111 / 1984 / 2194."""
     most = rows_per_group + 3 * rows_per_group ** 0.5
     if rows_per_group >= WT_MAX_ROWS:
         return 0
@@ -117,12 +117,14 @@ def grouped_gemm_bf16(a: torch.Tensor, b: torch.Tensor, group_offsets: torch.Ten
     up to 255 unused rows instead of up to 127). ``pair="wide"``: CTA pairs with 256 x 512 tiles, another quarter less
     traffic per FLOP, which is what raises the clock under the power limit. ``pair="swap"``: CTA pairs with the operands
     swapped (weight rows on the M side of the MMA, the tokens of a group on the N side in steps of 16): nothing is computed
-    for rows that do not exist, and a group of up to 256 rows passes over its weights once. ``tile_n`` (single CTAs only): tile width 128,
+    for rows that do not exist, and a group of up to 256 rows passes over its weights once; for deep products (K of 1536 and
+    more), since its epilogue is the longest. ``tile_n`` (single CTAs only): tile width 128,
     192 or 224 instead of 256, see :func:`pick_grouped_tile_n`. ``w_prefetch`` (single CTAs only): the producer asks L2 for
     the weight boxes this many 64-deep K blocks ahead of its loads, meant for launches that stream weights from HBM (few rows per
     group); measured slower than no prefetch at every distance on this part, so nothing sets it. ``tile_m=64`` (single CTAs, 256-wide
     tiles): row tiles of 64 instead of 128, for groups of a few dozen rows (a decode step): the A part of a pipeline stage
-    halves and the ring gets a fifth stage, so more weight bytes are in flight per SM. ``tile_tokens`` (64, 128 or 192; excludes
+    halves and the ring gets a fifth stage, so more weight bytes are in flight per SM; ``tile_tokens=64`` is the faster form of
+    such a launch, this one remains for callers that keep the tokens on the M side. ``tile_tokens`` (64, 128 or 192; excludes
     the other tile options): weights on the M side of the MMA, all rows of a group (cut into equal parts above ``tile_tokens``)
     on the N side: the form for launches that stream weights, see :func:`pick_tile_tokens`. ``chained`` (with ``tile_tokens``):
     the launch is scheduled while the kernel in front of it in the stream drains; 2 = ``group_offsets`` and ``b`` were
