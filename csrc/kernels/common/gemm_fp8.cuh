@@ -366,10 +366,10 @@ gemm_fp8_blockscaled_kernel(const __grid_constant__ CUtensorMap tmA, const __gri
             for (int kb = 0; kb < kblocks; ++kb) {
                 const float s = s_next;
                 if (kb + 1 < kblocks) s_next = sa_row[kb + 1] * sb_row[kb + 1];
-                // No vote here, once per K block: it costs 3-5 % of the kernel (1024 x 4096 x 7168: 38.1 -> 39.9 us). A lane whose wait ran
-                // out waits no more and goes on beside the others, so that tcgen05.ld below is reached by all of them; the vote
-                // is at the end of the tile.
-                if (ok) ok = mbar_wait(&pfull_bar[part], part_phase, st, 4, part, lim);
+                // No vote and no flag here, once per K block: either costs 3-5 % of a kernel that has no register left (1024 x 4096 x
+                // 7168: 38.1 -> 39.9 us). A lane whose wait ran out says so in the top bit of its phase, waits no more and goes on
+                // beside the others, so that tcgen05.ld below is reached by all of them; the vote is at the end of the tile.
+                if (static_cast<int>(part_phase) >= 0 && !mbar_wait(&pfull_bar[part], part_phase, st, 4, part, lim)) part_phase |= 1u << 31;
                 tc_fence_after_sync();
                 const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + part * kF8PartStride + grp * kF8Cols;
 #pragma unroll
@@ -387,7 +387,7 @@ gemm_fp8_blockscaled_kernel(const __grid_constant__ CUtensorMap tmA, const __gri
                     part_phase ^= 1;
                 }
             }
-            ok = __all_sync(0xffffffffu, ok);
+            ok = __all_sync(0xffffffffu, static_cast<int>(part_phase) >= 0);
             if (!ok) break;
             const int col0 = nt * kF8BN + grp * kF8Cols;
             if (valid) {

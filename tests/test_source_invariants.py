@@ -82,7 +82,7 @@ def test_waits_of_whole_warps_end_alike_in_all_lanes():
             if re.search(rf"(mbar_wait\w*|wait_flag_ge)\(.*\bst, ({places}),", line):
                 voted = "__all_sync" in line or re.search(r"mbar_wait\w*_warp\(", line)
                 # or the lane goes on without leaving the loop, and the vote comes at its end
-                kept = re.match(r"\s*if \(ok\) ok = mbar_wait\(", line) and any("ok = __all_sync(0xffffffffu, ok);" in t for t in lines[i: i + 30])
+                kept = "part_phase |= 1u << 31;" in line and any("ok = __all_sync(0xffffffffu, static_cast<int>(part_phase) >= 0);" in t for t in lines[i: i + 30])
                 if not voted and not kept and not any("epi_fail" in t for t in lines[i: i + 8]):
                     bad.append((p.name, i + 1))
     assert not bad, bad
