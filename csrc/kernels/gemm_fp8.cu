@@ -57,26 +57,37 @@ int ksplit_clusters(int size)
 // many CTAs as still run at the same time, if that shortens each CTA's run by 14 blocks: meeting twice and adding the sums
 // costs about 6 us (2000 x 544 x 1024: 20.5 us in clusters, 14.3 without). Else, with more than one row tile, CTA pairs: the r tiles that are left over after
 // the last full round are cut into the most column parts (2, 4 or 8) that still have a pair each, since a last round of few
-// wide tiles would take as long as a full one. The rest (one row tile, very wide) stays on single CTAs,
-// and so do all-gathered operands, whose order and pace are set by the arriving shards.
+// wide tiles would take as long as a full one. Where there is nothing to cut, single CTAs have as many rounds as pairs, and for a few
+// rounds of a deep product they are the faster ones: 1024 x 4096 x 7168 (one round) 38.1 us against 40.2 on pairs, x 4096 25.2 / 25.4,
+// 1500 x 8192 x 7168 (three rounds) 111 / 116, x 4096 71 / 70; with 3.9 rounds 153 / 153. One row tile and all-gathered
+// operands, whose order and pace are set by the arriving shards, stay on single CTAs too.
 int launch_plain_f8(const void* Aq, const void* Bq, const F8Args& g, long long lda, long long ldb, cudaStream_t stream)
 {
-    static bool pairs_configured[64] = {}, clusters_configured[64] = {};
-    SLIME_CUDA_OK(allow_dynamic_smem(gemm_fp8_pair_kernel, kF8pSmem, pairs_configured));
-    SLIME_CUDA_OK(allow_dynamic_smem(gemm_fp8_ksplit_kernel, kF8pSmem, clusters_configured));
     F8PairArgs f{};
     f.M = g.M, f.N = g.N, f.K = g.K, f.C = g.C, f.ldc = g.ldc, f.sa = g.sa, f.sb = g.sb, f.status = g.ag.status, f.wait_ns = g.ag.wait_ns;
     const int  sms     = sm_count();
     const long ntiles  = (f.N + kF8BN - 1) / kF8BN;
     const long tiles   = static_cast<long>((f.M + kBM - 1) / kBM) * ntiles;
     const int  kblocks = f.K / kF8BK;
+    const int  pairs   = sms / 2;
+    const long pair_tiles = static_cast<long>((f.M + 2 * kBM - 1) / (2 * kBM)) * ntiles;
+    const long rest       = pair_tiles % pairs;
+    int split = 1, parts = 1;
+    if (4 * tiles <= sms) {
+        static bool configured[64] = {};
+        SLIME_CUDA_OK(allow_dynamic_smem(gemm_fp8_ksplit_kernel, kF8pSmem, configured));
+        for (int c : {2, 4, 8})
+            if (kblocks - kblocks / c >= 14 && tiles <= ksplit_clusters(c)) split = c;
+    }
+    while (parts < 8 && rest > 0 && rest * parts * 2 <= pairs) parts *= 2;
+    if (split == 1) {
+        if (reinterpret_cast<unsigned long long>(f.C) % 16 != 0) return fail("fp8 gemm: the output must be 16-byte aligned (%p)", static_cast<void*>(f.C));
+        const bool few_rounds = parts == 1 && (pair_tiles <= pairs ? kblocks >= 36 : pair_tiles <= 3 * pairs && kblocks >= 44);
+        if (f.M <= kBM || few_rounds) return launch_f8<false>(Aq, Bq, nullptr, g, lda, ldb, stream);
+    }
     CUtensorMap tmA, tmB, tmBn;
     if (make_tmap_2d(&tmA, Aq, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, f.M, f.K, lda, kBM, kF8BK)) return -1;
     if (make_tmap_2d(&tmB, Bq, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, f.N, f.K, ldb, kF8BN / 2, kF8BK)) return -1;
-    int split = 1;
-    if (4 * tiles <= sms)
-        for (int c : {2, 4, 8})
-            if (kblocks - kblocks / c >= 14 && tiles <= ksplit_clusters(c)) split = c;
     cudaLaunchConfig_t cfg{};
     cfg.blockDim         = dim3(kF8pThreads);
     cfg.dynamicSmemBytes = kF8pSmem;
@@ -97,15 +108,10 @@ int launch_plain_f8(const void* Aq, const void* Bq, const F8Args& g, long long l
         SLIME_CUDA_OK(cudaLaunchKernelEx(&cfg, gemm_fp8_ksplit_kernel, tmA, tmB, f));
         return 0;
     }
-    if (reinterpret_cast<unsigned long long>(f.C) % 16 != 0) return fail("fp8 gemm: the output must be 16-byte aligned (%p)", static_cast<void*>(f.C));
-    if (f.M <= kBM) return launch_f8<false>(Aq, Bq, nullptr, g, lda, ldb, stream);
-    const int  pairs      = sms / 2;
-    const long pair_tiles = static_cast<long>((f.M + 2 * kBM - 1) / (2 * kBM)) * ntiles;
-    const long rest       = pair_tiles % pairs;
-    f.full_tiles          = static_cast<int>(pair_tiles);
-    f.split               = 1;
-    while (f.split < 8 && rest > 0 && rest * f.split * 2 <= pairs) f.split *= 2;
-    if (f.split > 1) f.full_tiles = static_cast<int>(pair_tiles - rest);
+    static bool configured[64] = {};
+    SLIME_CUDA_OK(allow_dynamic_smem(gemm_fp8_pair_kernel, kF8pSmem, configured));
+    f.split      = parts;
+    f.full_tiles = static_cast<int>(parts > 1 ? pair_tiles - rest : pair_tiles);
     const int widest = f.full_tiles > 0 ? kF8BN : kF8BN / f.split;
     f.stage_bytes    = kF8pABytes + widest / 2 * kF8BK;
     f.stages         = kF8pRingBytes / f.stage_bytes < kF8pMaxStages ? kF8pRingBytes / f.stage_bytes : kF8pMaxStages;

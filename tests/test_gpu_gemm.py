@@ -349,3 +349,10 @@ def test_clusters_are_worth_more_k_blocks_for_taller_tiles(m, k, shared):
 
     assert (_lib.call("slime_gemm_bf16_clusters", m, 2048, k) > 1) is shared
     test_gemm_bf16_few_tiles_share_k(m, 2048, k)
+
+
+@pytest.mark.parametrize("m,n,k", [(300, 8192, 4480), (300, 8192, 4608), (600, 3584, 4608), (701, 4320, 6912), (1000, 8192, 5632), (2300, 6144, 5760), (3000, 6144, 5632)])
+def test_gemm_fp8_deep_products_of_few_rounds(m, n, k):
+    """On both sides of the line between CTA pairs and single CTAs: one round below and from 36 K blocks, two and three rounds from 44, four
+    rounds; ragged rows and columns."""
+    test_gemm_fp8_forms(m, n, k)
