@@ -7,6 +7,7 @@
     python bench/profile_case.py grouped_pair  # grouped SwiGLU gate/up + down GEMM on CTA pairs, 8 experts x 1024 rows, 2 launches each
     python bench/profile_case.py grouped_decode  # gate/up GEMM of a decode step on 8 ranks (32 experts x 32 rows): 128-row tiles, then 64-row tiles with five stages
     python bench/profile_case.py gemm_fp8    # the same shape in block-scaled fp8 (e4m3), 3 launches
+    python bench/profile_case.py gemm_few    # 72 x 4096 x 7168 in bf16 and in block-scaled fp8: clusters that share each tile's K, 2 launches each
     python bench/profile_case.py grouped     # grouped SwiGLU gate/up + down GEMM, 8 experts x 512 rows, 2 launches each
     python bench/profile_case.py grouped_stream  # the same GEMMs with 16 experts x 128 rows: weight streaming, HBM-bound
     python bench/profile_case.py moe_step    # one single-GPU MoE layer step (T=1024, 32 experts of the 7168/2048 shape)
@@ -98,6 +99,18 @@ def gemm_fp8_case():
     out = torch.empty(4096, 4096, device="cuda", dtype=torch.bfloat16)
     for _ in range(3):
         gemm.gemm_fp8_blockscaled(aq, sa, bq, sb, out=out)
+
+
+def gemm_few_case():
+    from dlslime_b200.ops import gemm, quant
+
+    a = torch.randn(72, 7168, device="cuda").to(torch.bfloat16)
+    b = (torch.randn(4096, 7168, device="cuda") * 0.02).to(torch.bfloat16)
+    q, s = quant.fp8_quant_1x128(a)
+    w = quant.fp8_quant_128x128(b)
+    for _ in range(2):
+        gemm.gemm_bf16(a, b)
+        gemm.gemm_fp8_blockscaled(q, s, *w)
 
 
 def grouped_case():
@@ -266,6 +279,6 @@ def moe_stream_case():
 if __name__ == "__main__":
     {"ag_gemm_fused": ag_gemm_fused_case, "ag_gemm_fp8_fused": ag_gemm_fp8_fused_case, "moe_stream": moe_stream_case,
      "alltoall": alltoall_case, "kv": kv_case, "allgather": allgather_case, "gemm": gemm_case, "gemm_pair": gemm_pair_case, "gemm_wide": gemm_wide_case,
-     "grouped_pair": grouped_pair_case, "grouped_decode": grouped_decode_case, "gemm_fp8": gemm_fp8_case, "grouped": grouped_case, "grouped_stream": grouped_stream_case, "moe_step": moe_case, "quant": quant_case, "copy": copy_case}[sys.argv[1]]()
+     "grouped_pair": grouped_pair_case, "grouped_decode": grouped_decode_case, "gemm_fp8": gemm_fp8_case, "gemm_few": gemm_few_case, "grouped": grouped_case, "grouped_stream": grouped_stream_case, "moe_step": moe_case, "quant": quant_case, "copy": copy_case}[sys.argv[1]]()
     torch.cuda.synchronize()
     print("done", sys.argv[1])
