@@ -53,6 +53,9 @@ int slime_fp8_quant_128x128(const void* w, void* q, float* scales, int rows, int
 
 // ---- tcgen05 GEMMs (gemm.cu) -----------------------------------------------
 // C[M,N] = A[M,K] * B[N,K]^T, bf16 in, fp32 accumulate, bf16 out.
+// slime_gemm_bf16 if it shares K over clusters for this size, otherwise nothing is launched and 1 is returned
+int slime_gemm_bf16_few(const void* A, const void* B, void* C, int M, int N, int K, long long lda, long long ldb,
+                        long long ldc, void* status, void* stream);
 int slime_gemm_bf16_clusters(int M, int N, int K);  // CTAs per tile that slime_gemm_bf16 would share K over (1: no cluster)
 int slime_gemm_bf16(const void* A, const void* B, void* C, int M, int N, int K, long long lda, long long ldb,
                     long long ldc, void* status, void* stream);

@@ -366,6 +366,15 @@ int slime_gemm_bf16(const void* A, const void* B, void* C, int M, int N, int K, 
     return launch<kEpiStore>(A, B, a, lda, ldb, static_cast<cudaStream_t>(stream));
 }
 
+// slime_gemm_bf16 if it would share each tile's K over a cluster (see pick_ksplit); otherwise launches nothing and returns 1, so
+// that the caller takes another form without having asked first.
+int slime_gemm_bf16_few(const void* A, const void* B, void* C, int M, int N, int K, long long lda, long long ldb,
+                        long long ldc, void* status, void* stream)
+{
+    if (M > 0 && N > 0 && K > 0 && pick_ksplit(M, N, K) == 1) return 1;
+    return slime_gemm_bf16(A, B, C, M, N, K, lda, ldb, ldc, status, stream);
+}
+
 // The same product on CTA pairs (256-row tiles, tcgen05 cta_group::2).
 int slime_gemm_bf16_pair(const void* A, const void* B, void* C, int M, int N, int K, long long lda, long long ldb,
                          long long ldc, void* status, void* stream)

@@ -37,6 +37,7 @@ _SIGNATURES = {
     "slime_fp8_dequant_1x128": [c_void_p, c_void_p, c_void_p, c_longlong, c_int, c_longlong, c_longlong, c_void_p],
     "slime_fp8_quant_128x128": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_longlong, c_longlong, c_void_p],
     "slime_gemm_bf16_clusters": [c_int, c_int, c_int],
+    "slime_gemm_bf16_few": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_longlong, c_longlong, c_longlong, c_void_p, c_void_p],
     "slime_gemm_bf16": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_longlong, c_longlong, c_longlong, c_void_p, c_void_p],
     "slime_gemm_bf16_pair": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_longlong, c_longlong, c_longlong, c_void_p, c_void_p],
     "slime_gemm_fp8_blockscaled": [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_longlong, c_longlong,

@@ -57,8 +57,13 @@ def gemm_bf16(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor | None = None,
     if out is None:
         out = torch.empty((m, n), dtype=torch.bfloat16, device=a.device)
     if pair is None:
-        # two SMs per 256-row tile pay off as soon as there is a full tile, unless the launcher would share a deep product's K
-        pair = m >= 256 and not (k >= 2048 and _lib.call("slime_gemm_bf16_clusters", m, n, k) > 1)
+        # Two SMs per 256-row tile pay off as soon as there is a full tile, unless the launcher shares a deep product's K over
+        # clusters. It has the rule; 64 tiles, a quarter of more SMs than there are, only spare the call.
+        pair = m >= 256
+        if pair and k >= 2048 and -(-m // 128) * -(-n // 256) <= 64:
+            if _lib.call("slime_gemm_bf16_few", ptr(a), ptr(b), ptr(out), m, n, k, a.stride(0), b.stride(0), out.stride(0),
+                         default_status().dev_ptr, stream_ptr()) == 0:
+                return out
     if pair:
         return gemm_bf16_pair(a, b, out)
     _lib.call("slime_gemm_bf16", ptr(a), ptr(b), ptr(out), m, n, k, a.stride(0), b.stride(0), out.stride(0),

@@ -70,23 +70,31 @@ def test_autotune_times_every_form_on_request(monkeypatch):
     assert layer.timed == [False, True, "wide", "swap", "streamed"]
 
 
-@pytest.mark.parametrize("clusters,m,k,entry", [(4, 500, 7168, "slime_gemm_bf16"), (1, 500, 7168, "slime_gemm_bf16_pair"), (4, 500, 1024, "slime_gemm_bf16_pair"),
-                                                (4, 255, 1024, "slime_gemm_bf16"), (1, 72, 7168, "slime_gemm_bf16")])
-def test_products_of_few_tiles_follow_the_launchers_rule(monkeypatch, clusters, m, k, entry):
-    """gemm_bf16 asks the launcher whether it would share a tile's K over a cluster; where it would not (clusters that do not fit, a
-    smaller device) a product with a full 256-row tile goes to CTA pairs."""
+@pytest.mark.parametrize("shared,m,k,entries", [
+    (True, 500, 7168, ["slime_gemm_bf16_few"]), (False, 500, 7168, ["slime_gemm_bf16_few", "slime_gemm_bf16_pair"]),
+    (True, 500, 1024, ["slime_gemm_bf16_pair"]), (True, 255, 1024, ["slime_gemm_bf16"]), (False, 72, 7168, ["slime_gemm_bf16"]),
+    (False, 1025, 7168, ["slime_gemm_bf16_pair"])])
+def test_products_of_few_tiles_follow_the_launchers_rule(monkeypatch, shared, m, k, entries):
+    """gemm_bf16 leaves it to the launcher whether a tile's K is shared over a cluster; where it is not (clusters that do not fit, a
+    smaller device) a product with a full 256-row tile goes to CTA pairs. Products of many tiles do not ask."""
     import torch
 
     from dlslime_b200.ops import gemm
 
     calls = []
+
+    def call(name, *args):
+        calls.append(name)
+        return int(name == "slime_gemm_bf16_few" and not shared)
+
     monkeypatch.setattr(gemm, "require_cuda", lambda *t: None)
     monkeypatch.setattr(gemm, "ptr", lambda t: 0)
     monkeypatch.setattr(gemm, "stream_ptr", lambda *a: 0)
     monkeypatch.setattr(gemm, "default_status", lambda: type("S", (), {"dev_ptr": 0}))
-    monkeypatch.setattr(gemm._lib, "call", lambda name, *a: clusters if name == "slime_gemm_bf16_clusters" else calls.append(name))
-    gemm.gemm_bf16(torch.empty(m, k, dtype=torch.bfloat16), torch.empty(2048, k, dtype=torch.bfloat16))
-    assert calls == [entry]
+    monkeypatch.setattr(gemm._lib, "call", call)
+    a, b = torch.empty(m, k, dtype=torch.bfloat16), torch.empty(2048, k, dtype=torch.bfloat16)
+    assert gemm.gemm_bf16(a, b).shape == (m, 2048)
+    assert [c.replace("_wide", "_pair") for c in calls] == entries
 
 
 @pytest.mark.parametrize("world,fuse,thin,trace,names", [
