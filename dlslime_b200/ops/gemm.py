@@ -6,6 +6,8 @@ Weights use the ``nn.Linear`` layout ``[N, K]`` (K contiguous), activations are
 
 from __future__ import annotations
 
+import functools
+
 import torch
 
 from .. import _lib
@@ -13,6 +15,11 @@ from ._common import default_status, ptr, require_cuda, stream_ptr
 
 EPI_STORE, EPI_SWIGLU, EPI_SCATTER_ROWS = 0, 1, 2
 WT_MAX_ROWS, SWAP_MAX_ROWS = 176, 320  # rows per group up to which tile_tokens and pair="swap" are the faster forms
+
+
+@functools.cache
+def _sms(device: torch.device) -> int:
+    return torch.cuda.get_device_properties(device).multi_processor_count
 
 
 def _wide_tiles_pay(m: int, n: int, sms: int = 148) -> bool:
@@ -58,9 +65,9 @@ def gemm_bf16(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor | None = None,
         out = torch.empty((m, n), dtype=torch.bfloat16, device=a.device)
     if pair is None:
         # Two SMs per 256-row tile pay off as soon as there is a full tile, unless the launcher shares a deep product's K over
-        # clusters. It has the rule; 64 tiles, a quarter of more SMs than there are, only spare the call.
+        # clusters. The rule is the launcher's; a product of more tiles than it looks at only spares the call, 6 us of the host.
         pair = m >= 256
-        if pair and k >= 2048 and -(-m // 128) * -(-n // 256) <= 64:
+        if pair and k >= 2048 and -(-m // 128) * -(-n // 256) * 4 <= _sms(a.device):
             if _lib.call("slime_gemm_bf16_few", ptr(a), ptr(b), ptr(out), m, n, k, a.stride(0), b.stride(0), out.stride(0),
                          default_status().dev_ptr, stream_ptr()) == 0:
                 return out

@@ -73,7 +73,7 @@ def test_autotune_times_every_form_on_request(monkeypatch):
 @pytest.mark.parametrize("shared,m,k,entries", [
     (True, 500, 7168, ["slime_gemm_bf16_few"]), (False, 500, 7168, ["slime_gemm_bf16_few", "slime_gemm_bf16_pair"]),
     (True, 500, 1024, ["slime_gemm_bf16_pair"]), (True, 255, 1024, ["slime_gemm_bf16"]), (False, 72, 7168, ["slime_gemm_bf16"]),
-    (False, 1025, 7168, ["slime_gemm_bf16_pair"])])
+    (True, 513, 7168, ["slime_gemm_bf16_pair"])])
 def test_products_of_few_tiles_follow_the_launchers_rule(monkeypatch, shared, m, k, entries):
     """gemm_bf16 leaves it to the launcher whether a tile's K is shared over a cluster; where it is not (clusters that do not fit, a
     smaller device) a product with a full 256-row tile goes to CTA pairs. Products of many tiles do not ask."""
@@ -88,6 +88,7 @@ def test_products_of_few_tiles_follow_the_launchers_rule(monkeypatch, shared, m,
         return int(name == "slime_gemm_bf16_few" and not shared)
 
     monkeypatch.setattr(gemm, "require_cuda", lambda *t: None)
+    monkeypatch.setattr(gemm, "_sms", lambda device: 148)
     monkeypatch.setattr(gemm, "ptr", lambda t: 0)
     monkeypatch.setattr(gemm, "stream_ptr", lambda *a: 0)
     monkeypatch.setattr(gemm, "default_status", lambda: type("S", (), {"dev_ptr": 0}))
